@@ -792,7 +792,7 @@ def main():
             "e2e": {"value": e2e_v, "unit": METRIC, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
         }
         if mode == "faithful":
-            r["arithmetic"] = "faithful quotients and fused multiply-adds (VF_ARITH_FAITHFUL)"
+            r["arithmetic"] = "fused multiply-adds in the face fluxes (VF_ARITH_FAITHFUL)"
         if dt == "f32":
             r["near_dry_division"] = ("the Float64 quotient's bits (correctly rounded Float32 division) where "
                                       "|h| < 2 kappa" if mode != "no_near_dry" else "fast reciprocal everywhere")

@@ -142,13 +142,12 @@ int vf_step(vf_handle* h, double max_dt, double t, double* dt_out);
 /* Float64 arithmetic of the per-step kernels (vf_step, vf_simulate and the
  * wide members of a batch). VF_ARITH_REFERENCE (the default): every operation
  * rounds as the reference's Julia code does, so results equal the reference
- * CPU path bit for bit. VF_ARITH_FAITHFUL: quotients correct to about one ulp
- * (a refined hardware reciprocal shared by quotients with one divisor),
- * library cube roots and fused multiply-adds; the same passes and branches,
- * held to the 1e-12 relative max-norm tolerance against the reference path
- * instead of to its bits, and fewer FP64 instructions per cell. Stands in for
- * nothing in the reference (whose CPU and KernelAbstractions backends both
- * round every operation); VF_EINVAL for Float32 handles or another mode. */
+ * CPU path bit for bit. VF_ARITH_FAITHFUL: the face fluxes use fused
+ * multiply-adds; the same passes and branches, held to the 1e-12 relative
+ * max-norm tolerance against the reference path instead of to its bits, and
+ * fewer FP64 instructions per cell. Stands in for nothing in the reference
+ * (whose CPU and KernelAbstractions backends both round every operation);
+ * VF_EINVAL for Float32 handles or another mode. */
 #define VF_ARITH_REFERENCE 0
 #define VF_ARITH_FAITHFUL 1
 int vf_set_arithmetic(vf_handle* h, int32_t mode);
@@ -201,12 +200,16 @@ int vf_time_kernels(vf_handle* h, int64_t n_steps, float* ms_flux, float* ms_sta
  * returns either way. No reference counterpart (failure-detection test hook). */
 int vf_selftest_tile_wait(int32_t device, int32_t arrive, int32_t iterations, int32_t* gave_up);
 
-/* Self-test of the Float64 quotient every Float64 kernel uses (correctly
- * rounded reciprocals shared by a divisor's quotients, with the IEEE division
- * for the operands the method excludes): q[i] = a[i] / b[i] for n host
- * pairs, computed on the device. It must equal IEEE division bit for bit. No
- * reference counterpart (test hook). */
+/* Self-test of the Float64 quotient every Float64 kernel uses (computed in
+ * integers, with the IEEE division for the operands the method excludes):
+ * q[i] = a[i] / b[i] for n host pairs, computed on the device. It must equal
+ * IEEE division bit for bit. No reference counterpart (test hook). */
 int vf_selftest_quotients(int32_t device, const double* a, const double* b, int32_t n, double* q);
+
+/* Self-test of the Float64 roots of the same kernels: sq[i] = sqrt(x[i]) and
+ * cb[i] = cbrt(x[i]) for n host values, computed on the device; both are the
+ * correctly rounded roots. No reference counterpart (test hook). */
+int vf_selftest_roots(int32_t device, const double* x, int32_t n, double* sq, double* cb);
 
 /* Self-test of the near-dry velocity quotient of the Float32 kernels (face
  * sides and cells with |h| below the near-dry threshold divide (hu, hv) by

@@ -129,7 +129,10 @@ void fill_phys(const vf_handle* h, vf::Phys<T>& p) {
   p.dy = (T)dy;
   int ex = 0;
   p.dx_pow2 = std::frexp(dx, &ex) == 0.5 ? 1 : 0;
+  p.dx_exp = 1 - ex;
   p.dy_pow2 = std::frexp(dy, &ex) == 0.5 ? 1 : 0;
+  p.dy_exp = 1 - ex;
+  p.unit_rho = (T)c.rho == (T)1 ? 1 : 0;
   p.Cz = (T)c.friction_Cz;
   // Float32: velocities of cells and faces with |h| < VF_NEAR_DRY_FACTOR *
   // desingularizing_kappa (the depth scale of the desingularised division,
@@ -793,6 +796,22 @@ int vf_selftest_quotients(int32_t device, const double* a, const double* b, int3
   if (e == cudaSuccess) e = cudaMemcpy(q, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
   cudaFree(d);
   if (e != cudaSuccess) return cuda_fail(nullptr, e, "quotient self-test");
+  return VF_OK;
+}
+
+int vf_selftest_roots(int32_t device, const double* x, int32_t n, double* sq, double* cb) {
+  if (!x || !sq || !cb || n < 1) return fail(nullptr, VF_EINVAL, "x, sq, cb must be non-NULL and n >= 1");
+  cudaError_t e = cudaSetDevice(device);
+  if (e != cudaSuccess) return cuda_fail(nullptr, e, "cudaSetDevice");
+  double* d = nullptr;
+  const size_t bytes = sizeof(double) * (size_t)n;
+  if ((e = cudaMalloc(&d, 3 * bytes)) != cudaSuccess) return cuda_fail(nullptr, e, "cudaMalloc");
+  e = cudaMemcpy(d, x, bytes, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = vf::launch_selftest_roots(d, n, d + n, d + 2 * (size_t)n, nullptr);
+  if (e == cudaSuccess) e = cudaMemcpy(sq, d + n, bytes, cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(cb, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  if (e != cudaSuccess) return cuda_fail(nullptr, e, "root self-test");
   return VF_OK;
 }
 

@@ -141,6 +141,9 @@ __device__ __forceinline__ Phys<Dual<T>> dual_phys(const Phys<T>& p) {
   q.dy = p.dy;
   q.dx_pow2 = p.dx_pow2;
   q.dy_pow2 = p.dy_pow2;
+  q.dx_exp = p.dx_exp;
+  q.dy_exp = p.dy_exp;
+  q.unit_rho = p.unit_rho;
   q.Cz = p.Cz;
   q.near_dry = p.near_dry;
   q.friction = p.friction;

@@ -4,7 +4,7 @@
 #include "vf_step_impl.cuh"
 
 namespace vf {
-// a.arith == 1 hands the step to the faithful-quotient kernels of vf_f64f.cu.
+// a.arith == 1 hands the step to the tolerance-bound kernels of vf_f64f.cu.
 cudaError_t launch_step(const StepArgs<double>& a, const double* Uin, double* Uout, int parity, cudaStream_t st) {
   if (a.arith == 1) return vf_faithful_launch_step(&a, Uin, Uout, parity, st);
   return launch_step_impl<double>(a, Uin, Uout, parity, st);
@@ -57,6 +57,17 @@ static __global__ void k_selftest_quotients(const double* a, const double* b, in
 }
 cudaError_t launch_selftest_quotients(const double* a, const double* b, int n, double* q, cudaStream_t st) {
   k_selftest_quotients<<<(n + 255) / 256, 256, 0, st>>>(a, b, n, q);
+  return cudaGetLastError();
+}
+static __global__ void k_selftest_roots(const double* x, int n, double* sq, double* cb) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) {
+    sq[i] = Arith<double>::sqrt_(x[i]);
+    cb[i] = vcbrt<double>(x[i]);
+  }
+}
+cudaError_t launch_selftest_roots(const double* x, int n, double* sq, double* cb, cudaStream_t st) {
+  k_selftest_roots<<<(n + 255) / 256, 256, 0, st>>>(x, n, sq, cb);
   return cudaGetLastError();
 }
 

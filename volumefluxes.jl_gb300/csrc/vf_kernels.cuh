@@ -110,17 +110,17 @@ struct BTile {
   __device__ __forceinline__ T cn(int lx, int ly) const { return sB[(ly + 2) * BHX + lx + 2]; }
   __device__ __forceinline__ T cell(int lx, int ly) const {
     if (is_const) return c;
-    return (T)0.25 * (((cn(lx, ly) + cn(lx + 1, ly)) + cn(lx, ly + 1)) + cn(lx + 1, ly + 1));
+    return quarter<T>(((cn(lx, ly) + cn(lx + 1, ly)) + cn(lx, ly + 1)) + cn(lx + 1, ly + 1));
   }
   template <int DIR>
   __device__ __forceinline__ T face_l(int lx, int ly) const {
     if (is_const) return c;
-    return DIR == 0 ? (T)0.5 * (cn(lx, ly) + cn(lx, ly + 1)) : (T)0.5 * (cn(lx, ly) + cn(lx + 1, ly));
+    return halve<T>(DIR == 0 ? cn(lx, ly) + cn(lx, ly + 1) : cn(lx, ly) + cn(lx + 1, ly));
   }
   template <int DIR>
   __device__ __forceinline__ T face_r(int lx, int ly) const {
     if (is_const) return c;
-    return DIR == 0 ? (T)0.5 * (cn(lx + 1, ly) + cn(lx + 1, ly + 1)) : (T)0.5 * (cn(lx, ly + 1) + cn(lx + 1, ly + 1));
+    return halve<T>(DIR == 0 ? cn(lx + 1, ly) + cn(lx + 1, ly + 1) : cn(lx, ly + 1) + cn(lx + 1, ly + 1));
   }
 };
 
@@ -205,7 +205,7 @@ __device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, c
     sF[idx] = F0;
     sF[FN + idx] = F1;
     sF[2 * FN + idx] = F2;
-    if (SPEED && ly < nvy && f <= nvx) mx = fmax(mx, sp);
+    if (SPEED && ly < nvy && f <= nvx) mx = speed_max<T>(mx, sp);
   }
   __syncthreads();
   // ---- x: accumulate
@@ -214,12 +214,21 @@ __device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, c
     const int c = tid + k * NT;
     const int lx = c % TX, ly = c / TX;
     const int fl = ly * (TX + 1) + lx;
+    if constexpr (std::is_same<T, double>::value) {
+      T v[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) acc[k][j] = (T)0 - p.inv_dx * (sF[j * FN + fl + 1] - sF[j * FN + fl]);
+      for (int j = 0; j < 3; ++j) v[j] = sF[j * FN + fl + 1] - sF[j * FN + fl];
+      over_delta<0>(p, v);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[k][j] = exact::zero_minus(v[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[k][j] = (T)0 - p.inv_dx * (sF[j * FN + fl + 1] - sF[j * FN + fl]);
+    }
     const int rc = ly * (TX + 2) + lx + 1;
     for (int b = 0; b < p.n_bottom; ++b) {
       const T Bl = bt.template face_l<0>(lx, ly), Br = bt.template face_r<0>(lx, ly);
-      acc[k][1] = acc[k][1] + p.neg_g * slope_over<T>(Br - Bl, p.dx, p.inv_dx, p.dx_pow2) * ((sR[rc] + sL[rc]) * (T)0.5);
+      acc[k][1] = acc[k][1] + p.neg_g * bottom_slope<T, 0>(p, Br - Bl) * halve<T>(sR[rc] + sL[rc]);
     }
   }
   __syncthreads();
@@ -256,7 +265,7 @@ __device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, c
     sF[idx] = F0;
     sF[FN + idx] = F1;
     sF[2 * FN + idx] = F2;
-    if (SPEED && lx < nvx && f <= nvy) my = fmax(my, sp);
+    if (SPEED && lx < nvx && f <= nvy) my = speed_max<T>(my, sp);
   }
   __syncthreads();
   // ---- y: accumulate
@@ -265,12 +274,21 @@ __device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, c
     const int c = tid + k * NT;
     const int lx = c % TX, ly = c / TX;
     const int fl = ly * TX + lx;
+    if constexpr (std::is_same<T, double>::value) {
+      T v[3];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) acc[k][j] = acc[k][j] - p.inv_dy * (sF[j * FN + fl + TX] - sF[j * FN + fl]);
+      for (int j = 0; j < 3; ++j) v[j] = sF[j * FN + fl + TX] - sF[j * FN + fl];
+      over_delta<1>(p, v);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[k][j] = acc[k][j] - v[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[k][j] = acc[k][j] - p.inv_dy * (sF[j * FN + fl + TX] - sF[j * FN + fl]);
+    }
     const int rc = (ly + 1) * TX + lx;
     for (int b = 0; b < p.n_bottom; ++b) {
       const T Bl = bt.template face_l<1>(lx, ly), Br = bt.template face_r<1>(lx, ly);
-      acc[k][2] = acc[k][2] + p.neg_g * slope_over<T>(Br - Bl, p.dy, p.inv_dy, p.dy_pow2) * ((sR[rc] + sL[rc]) * (T)0.5);
+      acc[k][2] = acc[k][2] + p.neg_g * bottom_slope<T, 1>(p, Br - Bl) * halve<T>(sR[rc] + sL[rc]);
     }
   }
 }
@@ -351,7 +369,10 @@ __device__ __forceinline__ void flux_tile(const Geom<T>& g, const Phys<T>& p, co
     for (int j = 0; j < 3; ++j) Lout[j * g.PS + o] = acc[k][j];
     if (p.friction) {
       const int ci = (ly + 2) * HX + lx + 2;
-      Sout[o] = friction_factor<T>(p, s.U[ci], s.U[HX * HY + ci], s.U[2 * HX * HY + ci], bt.cell(lx, ly));
+      const T q0 = s.U[ci], q1 = s.U[HX * HY + ci], q2 = s.U[2 * HX * HY + ci];
+      // at rest the factor is a zero whatever the depth, and every reader skips
+      // zeros (Float32, bound by its registers here, computes it all the same)
+      Sout[o] = sizeof(T) == 4 || friction_active<T>(q1, q2) ? friction_factor<T>(p, q0, q1, q2, bt.cell(lx, ly)) : (T)0;
     }
   }
 }
@@ -756,9 +777,9 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
     T w = v0 + tdt * acc[k][0];
     T hu = v1 + tdt * acc[k][1];
     T hv = v2 + tdt * acc[k][2];
-    w = (T)0.5 * (s.U0[c] + w);
-    hu = (T)0.5 * (s.U0[TX * TY + c] + hu);
-    hv = (T)0.5 * (s.U0[2 * TX * TY + c] + hv);
+    w = halve<T>(s.U0[c] + w);
+    hu = halve<T>(s.U0[TX * TY + c] + hu);
+    hv = halve<T>(s.U0[2 * TX * TY + c] + hv);
     const T Bc = bt.cell(lx, ly);
     if (p.friction && friction_active<T>(v1, v2)) apply_friction<T>(tdt, friction_factor<T>(p, v0, v1, v2, Bc), hu, hv);
     dry_clamp<T>(p, w, hu, hv, Bc);

@@ -9,13 +9,17 @@
 //
 // GB300 executes Float64 at 1/64 of the Float32 rate, so the Float64 traits
 // below move every comparison, min/max and sign test onto the integer pipe by
-// comparing IEEE bit patterns; only +, -, *, /, sqrt stay on the FP64 pipe.
+// comparing IEEE bit patterns, and quotients, square roots and products with
+// powers of two by computing them in integers (vf_exact.h); only +, -, * stay
+// on the FP64 pipe.
 //
 // Citations are path:line within the VolumeFluxes.jl project.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
+#include "vf_exact.h"
 
 // Float32 reciprocals and cube roots come from the special-function unit
 // (rcp.approx, and cbrt(x) = 2^(log2|x| / 3) with the sign of x; a few ulps);
@@ -23,24 +27,12 @@
 // Measured on the 4096^2 wet/dry step (Float32 is instruction-issue bound):
 // 0.919 ms with the special-function unit, 1.069 ms with the correctly
 // rounded reciprocal and the libm cube root.
-// Float64 quotients correct to about one ulp instead of correctly rounded (1),
-// for the tolerance-bound Float64 kernels (vf_f64f.cu, built with multiply-add
-// contraction): a reciprocal from the hardware approximation refined by one
-// third-order Newton step, a quotient a/b as a * (1/b) plus one residual
-// correction, and quotients that share a divisor as products with one shared
-// reciprocal. Cube roots come from the CUDA math library. 0: every operation
-// rounds as in the reference (the bitwise kernels).
+// 1 (vf_f64f.cu): the tolerance-bound Float64 kernels, whose face fluxes use
+// fused multiply-adds. 0: every operation rounds as in the reference (the
+// bitwise kernels). Quotients, square roots and cube roots are the correctly
+// rounded ones of vf_exact.h in both: they cost no FP64 instructions.
 #ifndef VF_FP64_FAITHFUL
 #define VF_FP64_FAITHFUL 0
-#endif
-// Correctly rounded Float64 quotients from one correctly rounded reciprocal per
-// divisor (1) instead of one hardware IEEE division per quotient (0): the same
-// bits, fewer FP64 instructions where several quotients share a divisor. The
-// Float64 unit builds with 1: bit for bit the IEEE results on every parity
-// case and over the 4096^2 wet/dry workload's 1000 steps, and 28.8 instead of
-// 31.0 ms per step there (1.43x on the fully wet 256^2 dam break).
-#ifndef VF_FP64_MARKSTEIN
-#define VF_FP64_MARKSTEIN 0
 #endif
 
 namespace vf {
@@ -67,105 +59,26 @@ struct Arith<double> {
   }
   static __device__ __forceinline__ bool lt(double x, double y) { return key(x) < key(y) && !both_zero(x, y); }
   static __device__ __forceinline__ bool gt(double x, double y) { return key(x) > key(y) && !both_zero(x, y); }
-  static __device__ __forceinline__ bool gt0(double x) { return bits(x) > 0; }
-  static __device__ __forceinline__ bool lt0(double x) {
-    return (unsigned long long)bits(x) > 0x8000000000000000ull;
-  }
+  static __device__ __forceinline__ bool gt0(double x) { return __double2hiint(x) >= 0 && !exact::zero(x); }
+  static __device__ __forceinline__ bool lt0(double x) { return __double2hiint(x) < 0 && !exact::zero(x); }
   // |x| < k and |x| >= k for k >= 0.
   static __device__ __forceinline__ bool abs_lt(double x, double k) {
     return (unsigned long long)(bits(x) & 0x7fffffffffffffffll) < (unsigned long long)bits(k);
   }
-  static __device__ __forceinline__ bool is_zero(double x) { return (bits(x) << 1) == 0ll; }
+  static __device__ __forceinline__ bool is_zero(double x) { return exact::zero(x); }
   // Julia's max/min: -0.0 < +0.0.
   static __device__ __forceinline__ double max(double x, double y) { return key(x) > key(y) ? x : y; }
   static __device__ __forceinline__ double min(double x, double y) { return key(x) < key(y) ? x : y; }
-#if VF_FP64_FAITHFUL
-  // Reciprocal: the hardware approximation r0 (rcp.approx.ftz.f64, relative
-  // error e0) refined by one third-order Newton step r0 * (1 + e + e^2) with
-  // e = 1 - b*r0, whose error is e0^3 plus the rounding of the last fused
-  // multiply-add. Divisors on this path are normal numbers (desingularised
-  // depths >= kappa/2, wave-speed spreads >= kappa, 1 - dt*S >= 1).
-  static __device__ __forceinline__ double rcp(double b) {
-    double r0;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(b));
-    const double e = fma(-b, r0, 1.0);
-    return fma(r0, fma(e, e, e), r0);
-  }
-  // a/b as q = a * (1/b) corrected once by the exact residual a - b*q.
-  static __device__ __forceinline__ double div(double a, double b) {
-    const double r = rcp(b);
-    const double q = a * r;
-    return fma(fma(-b, q, a), r, q);
-  }
-  static __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
-  struct Recip {
-    double r;
-  };
-  static __device__ __forceinline__ Recip recip(double b) { return Recip{rcp(b)}; }
-  static __device__ __forceinline__ double div_by(const Recip& R, double a) { return a * R.r; }
-  static __device__ __forceinline__ double inv(const Recip& R) { return R.r; }
-#elif VF_FP64_MARKSTEIN
-  // Correctly rounded quotients through a correctly rounded reciprocal
-  // (Markstein, IBM J. Res. Dev. 34(1), 1990; Cornea, Harrison & Tang,
-  // Scientific Computing on Itanium-based Systems, ch. 8):
-  //  1. y1 = the hardware reciprocal refined by one third-order Newton step,
-  //     within one ulp of 1/b;
-  //  2. y = y1 + y1*(1 - b*y1) (two fused multiply-adds) is RN(1/b) for every b
-  //     whose significand is not all ones;
-  //  3. q0 = RN(a*y) is within one ulp of a/b, the residual a - b*q0 is exact
-  //     in one fused multiply-add, and RN(q0 + (a - b*q0)*y) is RN(a/b).
-  // The steps need normal operands with quotients far from overflow and
-  // underflow: a divisor with an all-ones significand or an exponent outside
-  // +-500 (zero, subnormal, infinite and NaN divisors included), or a nonzero
-  // numerator outside that range (infinite and NaN numerators included),
-  // takes the IEEE division. A zero numerator over an in-range divisor
-  // returns a*y, the correctly signed zero.
-  struct Recip {
-    double b, y;
-    bool ok;
-  };
-  static __device__ __forceinline__ bool mid_range(long long x) {
-    const int e = (int)((x >> 52) & 0x7ff);
-    return e > 1023 - 500 && e < 1023 + 500;
-  }
-  static __device__ __forceinline__ Recip recip(double b) {
-    const long long bb = bits(b);
-    double r0;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r0) : "d"(b));
-    const double e0 = fma(-b, r0, 1.0);
-    const double y1 = fma(r0, fma(e0, e0, e0), r0);
-    const double e1 = fma(-b, y1, 1.0);
-    return Recip{b, fma(y1, e1, y1), mid_range(bb) && (bb & 0xfffffffffffffll) != 0xfffffffffffffll};
-  }
-  static __device__ __forceinline__ double div_by(const Recip& R, double a) {
-    if (!R.ok) return a / R.b;
-    const double q0 = a * R.y;
-    if (is_zero(a)) return q0;
-    if (!mid_range(bits(a))) return a / R.b;
-    return fma(fma(-R.b, q0, a), R.y, q0);
-  }
+  // Correctly rounded quotients and square roots in integers (vf_exact.h):
+  // the IEEE bits without an FP64 instruction, about 55 integer and Float32
+  // instructions each.
+  using Recip = exact::Divisor;
+  static __device__ __forceinline__ Recip recip(double b) { return exact::divisor(b); }
+  static __device__ __forceinline__ double div_by(const Recip& R, double a) { return exact::quotient(R, a); }
   static __device__ __forceinline__ double div(double a, double b) { return div_by(recip(b), a); }
   static __device__ __forceinline__ double rcp(double b) { return div(1.0, b); }
-  // 1/b for terms that need no correct rounding (the derivative parts of
-  // dual numbers): the correctly rounded reciprocal, where the method applies.
-  static __device__ __forceinline__ double inv(const Recip& R) { return R.ok ? R.y : 1.0 / R.b; }
-  static __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
-#else
-  // Correctly rounded division and square root on the FP64 pipe, one IEEE
-  // division per quotient. (Measured on the 4096^2 wet/dry step and not kept:
-  // a correctly rounded division on the integer pipe, 40.0 vs 31.5 ms per
-  // step, and quotients sharing one refined reciprocal with a Float64 rounding
-  // test and a fallback, 41.1 vs 31.0 ms.)
-  static __device__ __forceinline__ double div(double a, double b) { return a / b; }
-  static __device__ __forceinline__ double rcp(double b) { return 1.0 / b; }
-  static __device__ __forceinline__ double sqrt_(double x) { return sqrt(x); }
-  struct Recip {
-    double b;
-  };
-  static __device__ __forceinline__ Recip recip(double b) { return Recip{b}; }
-  static __device__ __forceinline__ double div_by(const Recip& R, double a) { return a / R.b; }
-  static __device__ __forceinline__ double inv(const Recip& R) { return 1.0 / R.b; }
-#endif  // VF_FP64_FAITHFUL
+  static __device__ __forceinline__ double inv(const Recip& R) { return div_by(R, 1.0); }
+  static __device__ __forceinline__ double sqrt_(double x) { return exact::square_root(x); }
 };
 
 template <>
@@ -192,10 +105,10 @@ struct Arith<float> {
 };
 
 // ---------------------------------------------------------------------------
-// Correctly rounded cube root (Float64). A libm seed is corrected with an exact
-// integer comparison against the rounding midpoints, so the result is the
-// nearest double regardless of the seed's last-bit error; the CPU oracle
-// computes the same unique value.
+// Correctly rounded cube root (Float64). A seed within an ulp or two is
+// corrected with an exact integer comparison against the rounding midpoints, so
+// the result is the nearest double regardless of the seed's last-bit error; the
+// CPU oracle computes the same unique value.
 __device__ __forceinline__ void cube_u55(uint64_t k, uint64_t& w0, uint64_t& w1, uint64_t& w2) {
   const uint64_t lo = k * k, hi = __umul64hi(k, k);       // k^2 < 2^110
   const uint64_t p0lo = k * lo, p0hi = __umul64hi(k, lo);  // k*lo < 2^119
@@ -214,14 +127,12 @@ __device__ __forceinline__ int cmp192(uint64_t a0, uint64_t a1, uint64_t a2, uin
 // Out of line: the friction law calls it from two places per cell and step
 // (inlined it measured 31.06 vs 31.00 ms per 4096^2 wet/dry step).
 static __device__ __noinline__ double cr_cbrt(double x) {
-  if (x == 0.0 || !isfinite(x)) return x;
-  const bool neg = signbit(x);
-  double a = fabs(x);
+  const uint64_t sign = exact::bits(x) & 0x8000000000000000ull;
+  uint64_t bits = exact::bits(x) ^ sign;
+  if (bits == 0 || bits >= 0x7ff0000000000000ull) return x;
   int extra = 0;
-  uint64_t bits = (uint64_t)__double_as_longlong(a);
   if ((bits >> 52) == 0) {
-    a = a * 18014398509481984.0;  // 2^54, exact
-    bits = (uint64_t)__double_as_longlong(a);
+    bits = exact::bits(exact::from_bits(bits) * 18014398509481984.0);  // 2^54, exact
     extra = 18;
   }
   const int e = (int)(bits >> 52) - 1023;
@@ -230,14 +141,14 @@ static __device__ __noinline__ double cr_cbrt(double x) {
   const int q = e >= 0 ? e / 3 : -((-e + 2) / 3);
   const int r = e - 3 * q;  // 0, 1, 2
   const double t = __longlong_as_double((long long)(((uint64_t)(1023 + r) << 52) | frac));  // in [1, 8)
-  const double y0 = cbrt(t);
+  const uint64_t y0 = exact::bits(exact::cube_root_seed(t));
   uint64_t Y;
-  if (y0 >= 2.0) {
+  if (y0 >= 0x4000000000000000ull) {         // 2
     Y = 1ull << 53;
-  } else if (y0 < 1.0) {
+  } else if (y0 < 0x3ff0000000000000ull) {   // 1
     Y = 1ull << 52;
   } else {
-    Y = ((uint64_t)__double_as_longlong(y0) & ((1ull << 52) - 1)) | (1ull << 52);
+    Y = (y0 & ((1ull << 52) - 1)) | (1ull << 52);
   }
   // t * 2^159 = M * 2^(r + 107): limbs (0, M << (43 + r), M >> (21 - r)).
   const uint64_t T1 = M << (43 + r), T2 = M >> (21 - r);
@@ -255,16 +166,11 @@ static __device__ __noinline__ double cr_cbrt(double x) {
   int ex = q - extra;
   uint64_t mant = Y;
   if (mant == (1ull << 53)) { mant >>= 1; ex += 1; }
-  const double y = __longlong_as_double((long long)(((uint64_t)(ex + 1023) << 52) | (mant & ((1ull << 52) - 1))));
-  return neg ? -y : y;
+  return exact::from_bits(((uint64_t)(ex + 1023) << 52) | (mant & ((1ull << 52) - 1)) | sign);
 }
 
 template <typename T> __device__ __forceinline__ T vcbrt(T x);
-#if VF_FP64_FAITHFUL
-template <> __device__ __forceinline__ double vcbrt<double>(double x) { return cbrt(x); }
-#else
 template <> __device__ __forceinline__ double vcbrt<double>(double x) { return cr_cbrt(x); }
-#endif
 template <> __device__ __forceinline__ float vcbrt<float>(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__log2f(fabsf(x)) * (1.0f / 3.0f)));
@@ -276,6 +182,38 @@ template <typename T> __device__ __forceinline__ T jmax(T x, T y) { return Arith
 template <typename T> __device__ __forceinline__ T jmin(T x, T y) { return Arith<T>::min(x, y); }
 template <typename T> __device__ __forceinline__ T vdiv(T a, T b) { return Arith<T>::div(a, b); }
 
+// x/2 and x/4: for Float64 on the exponent field (the same bits).
+template <typename T> __device__ __forceinline__ T halve(T x) {
+  if constexpr (std::is_same<T, double>::value) return exact::half(x);
+  else return (T)0.5 * x;
+}
+template <typename T> __device__ __forceinline__ T quarter(T x) {
+  // halving twice rounds as a quarter does: x/2 is inexact only where its last
+  // place is the smallest there is, and rounds to even there
+  if constexpr (std::is_same<T, double>::value) return exact::half(exact::half(x));
+  else return (T)0.25 * x;
+}
+// a*b + c and a*b - c of the face fluxes: one rounding in the tolerance-bound
+// Float64 kernels, two (as the reference's) in the bitwise ones; other types
+// as their unit's contraction setting has it.
+template <typename T> __device__ __forceinline__ T madd(T a, T b, T c) {
+  if constexpr (std::is_same<T, double>::value && VF_FP64_FAITHFUL) return __fma_rn(a, b, c);
+  else return a * b + c;
+}
+template <typename T> __device__ __forceinline__ T msub(T a, T b, T c) {
+  if constexpr (std::is_same<T, double>::value && VF_FP64_FAITHFUL) return __fma_rn(a, b, -c);
+  else return a * b - c;
+}
+// The larger of two speeds >= 0, ignoring a NaN in v.
+template <typename T> __device__ __forceinline__ T speed_max(T m, T v) {
+  if constexpr (std::is_same<T, double>::value) {
+    const long long b = __double_as_longlong(v);
+    return b > __double_as_longlong(m) && b <= 0x7ff0000000000000ll ? v : m;
+  } else {
+    return fmax(m, v);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Physical constants of one simulation in the state's real type.
 template <typename T>
@@ -285,6 +223,8 @@ struct Phys {
   T inv_dx, inv_dy;           // 1/Δx, 1/Δy (src/numericalflux/numericalflux.jl:27)
   T dx, dy;                   // Δx, Δy (src/sourceterms/source_term_bottom.jl:38)
   int dx_pow2, dy_pow2;       // Δ is a power of two: x/Δ == x*(1/Δ) exactly
+  int dx_exp, dy_exp;         // then 1/Δ == 2^exp
+  int unit_rho;               // rho == 1: rho*h == h exactly
   T Cz;
   T near_dry;                 // Float32: |h| below this takes the Float64 velocity division (0: never)
   int friction;               // VF_FRICTION_*
@@ -363,6 +303,37 @@ __device__ __forceinline__ T slope_over(T dB, T delta, T inv_delta, int pow2) {
   return pow2 ? dB * inv_delta : Arith<T>::div(dB, delta);
 }
 
+// v[j] * (1/Δ) along DIR in Float64: for a power-of-two Δ on the exponent field
+// (nothing where Δ is 1), the same bits as the products.
+template <int DIR, int N>
+__device__ __forceinline__ void over_delta(const Phys<double>& p, double (&v)[N]) {
+  const double inv = DIR == 0 ? p.inv_dx : p.inv_dy;
+  if (DIR == 0 ? p.dx_pow2 : p.dy_pow2) {
+    const int k = DIR == 0 ? p.dx_exp : p.dy_exp;
+    if (k != 0) {
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = exact::scale_pow2(v[j], k, inv);
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < N; ++j) v[j] = exact::off_path_mul(inv, v[j]);
+}
+// The bottom source's slope ΔB/Δ along DIR in the tile kernels.
+template <typename T, int DIR>
+__device__ __forceinline__ T bottom_slope(const Phys<T>& p, T dB) {
+  if constexpr (std::is_same<T, double>::value) {
+    if (DIR == 0 ? p.dx_pow2 : p.dy_pow2) {
+      double v[1] = {dB};
+      over_delta<DIR>(p, v);
+      return v[0];
+    }
+    return Arith<T>::div(dB, DIR == 0 ? p.dx : p.dy);
+  } else {
+    return slope_over<T>(dB, DIR == 0 ? p.dx : p.dy, DIR == 0 ? p.inv_dx : p.inv_dy, DIR == 0 ? p.dx_pow2 : p.dy_pow2);
+  }
+}
+
 // Rain and infiltration in list order (src/system.jl:71-73), unrolled so the
 // parameter block is never indexed dynamically. `scal` holds point_scalars();
 // `cell` is the cell's offset in the state layout (for per-cell arrays).
@@ -375,9 +346,8 @@ __device__ __forceinline__ T add_point_sources(const Phys<T>& p, T acc0) {
   if constexpr (sizeof(T) == 4) {
     return acc0 + p.point_sum;
   } else {
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-      if (n < p.n_point) acc0 = acc0 + p.point_add[n];
+#pragma unroll 1
+    for (int n = 0; n < p.n_point; ++n) acc0 = acc0 + p.point_add[n];
     return acc0;
   }
 }
@@ -452,16 +422,21 @@ __device__ __forceinline__ void side_flux(const Phys<T>& p, T h, T hu, T hv, T& 
   const T hs = desing<T, SEL>(h, p.kappa);
   T u, v;
   velocities<T>(p, h, hs, hu, hv, u, v);
-  const T rh = p.rho * h;
+  T rh = h;
+  if constexpr (std::is_same<T, double>::value) {
+    if (!p.unit_rho) rh = exact::off_path_mul(p.rho, h);
+  } else {
+    rh = p.rho * h;
+  }
   const T hh = h * h;
   if (DIR == 0) {
     f0 = rh * u;
-    f1 = f0 * u + p.c2 * hh;
+    f1 = madd<T>(f0, u, p.c2 * hh);
     f2 = f0 * v;
   } else {
     f0 = rh * v;
     f1 = (rh * u) * v;
-    f2 = f0 * v + p.c2 * hh;
+    f2 = madd<T>(f0, v, p.c2 * hh);
   }
   const T c = A::sqrt_(p.g * h);
   const T un = DIR == 0 ? u : v;
@@ -489,9 +464,9 @@ __device__ __forceinline__ void cu_face(const Phys<T>& p, T mh, T mhu, T mhv, T 
   }
   const typename A::Recip R = A::recip(d);
   const T q = A::div_by(R, aplus * aminus);
-  F0 = A::div_by(R, aplus * fm0 - aminus * fp0) + q * (ph - mh);
-  F1 = A::div_by(R, aplus * fm1 - aminus * fp1) + q * (phu - mhu);
-  F2 = A::div_by(R, aplus * fm2 - aminus * fp2) + q * (phv - mhv);
+  F0 = madd<T>(q, ph - mh, A::div_by(R, msub<T>(aplus, fm0, aminus * fp0)));
+  F1 = madd<T>(q, phu - mhu, A::div_by(R, msub<T>(aplus, fm1, aminus * fp1)));
+  F2 = madd<T>(q, phv - mhv, A::div_by(R, msub<T>(aplus, fm2, aminus * fp2)));
   if (SPEED)
     speed = (A::lt(mh, p.cutoff) && A::lt(ph, p.cutoff)) ? (T)0 : A::max(fabs(aplus), fabs(aminus));
 }
@@ -521,6 +496,23 @@ __device__ __forceinline__ T minmod_slope(T l, T c, T r, T theta) {
   return minmod<T>(theta * fwd, central, theta * bwd);
 }
 
+// Half the minmod slope in Float64, minmod_slope's value times 0.5 bit for bit.
+// Rounding is monotone, so the smaller of theta*fwd and theta*bwd is theta
+// times the smaller difference: one product instead of two, and the halves and
+// the choice among operands of one sign (the smaller magnitude has the smaller
+// bits) are integer work. 4 FP64 instructions instead of 7.
+__device__ __forceinline__ double half_slope(double l, double c, double r, double theta) {
+  const double fwd = r - c, bwd = c - l;
+  const double mean = exact::half(fwd + bwd);
+  const unsigned long long bf = exact::bits(fwd), bb = exact::bits(bwd), bm = exact::bits(mean);
+  const double t = theta * exact::from_bits(bf < bb ? bf : bb);
+  const unsigned long long bt = exact::bits(t);
+  const bool one_sign = (long long)((bf ^ bb) | (bt ^ bm) | (bf ^ bm)) >= 0;  // all four alike
+  // with one sign, the smaller of t and mean is a zero when any of the four is
+  const double s = exact::from_bits(bt < bm ? bt : bm);
+  return one_sign && !exact::zero(s) ? exact::half(s) : 0.0;
+}
+
 // Practical-SWE linear reconstruction of one cell along one direction,
 // src/reconstruction/linearreconstruction.jl:73-100. Inputs are (w, hu, hv) at
 // the left, middle and right cells; outputs are face (h, hu, hv).
@@ -528,6 +520,27 @@ template <typename T>
 __device__ __forceinline__ void reconstruct_cell(const Phys<T>& p, const T l[3], const T c[3], const T r[3], T Bl, T Br,
                                                  T L[3], T R[3]) {
   using A = Arith<T>;
+  if constexpr (std::is_same<T, double>::value) {
+    // The same values with half slopes: 0.5 * (2 (w - Bl)) is w - Bl.
+    const double w = c[0];
+    const double h0 = half_slope(l[0], w, r[0], p.theta);
+    double wl = w - h0, wr = w + h0;
+    const bool below_l = A::lt(wl, Bl);
+    if (below_l || A::lt(wr, Br)) {
+      const double d = below_l ? w - Bl : Br - w;
+      wl = w - d;
+      wr = w + d;
+    }
+    L[0] = wl - Bl;
+    R[0] = wr - Br;
+#pragma unroll
+    for (int k = 1; k < 3; ++k) {
+      const double hs = half_slope(l[k], c[k], r[k], p.theta);
+      L[k] = c[k] - hs;
+      R[k] = c[k] + hs;
+    }
+    return;
+  }
   T s0 = minmod_slope<T>(l[0], c[0], r[0], p.theta);
   const T s1 = minmod_slope<T>(l[1], c[1], r[1], p.theta);
   const T s2 = minmod_slope<T>(l[2], c[2], r[2], p.theta);

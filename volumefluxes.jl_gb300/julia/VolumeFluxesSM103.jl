@@ -26,8 +26,8 @@ using VolumeFluxes: Simulator, ConservedSystem, CartesianGrid, WallBC, ShallowWa
 const LIB = get(ENV, "VF_SM103_LIB", joinpath(@__DIR__, "..", "volumefluxes_sm103", "lib", "libvfsm103.so"))
 
 # arithmetic (Float64 only): :reference rounds every operation as the reference
-# does (bitwise equal to its CPU path); :faithful uses faithful quotients and
-# fused multiply-adds (vf_set_arithmetic), held to a tolerance instead.
+# does (bitwise equal to its CPU path); :faithful uses fused multiply-adds in
+# the face fluxes (vf_set_arithmetic), held to a tolerance instead.
 struct SM103Backend{RealType} <: VolumeFluxes.Backend
     realtype::Type{RealType}
     device::Int32

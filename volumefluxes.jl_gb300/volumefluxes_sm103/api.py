@@ -436,7 +436,7 @@ class SM103Backend:
     `realtype` is np.float64 or np.float32, `device` a CUDA ordinal.
     `arithmetic` (Float64 only): "reference" rounds every operation as the
     reference does (results equal its CPU path bit for bit); "faithful" uses
-    faithful quotients and fused multiply-adds in the per-step kernels, held
+    fused multiply-adds in the face fluxes of the per-step kernels, held
     to 1e-12 relative max-norm against the reference path instead of to its
     bits.
     """
