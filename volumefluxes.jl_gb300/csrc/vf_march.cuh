@@ -65,9 +65,16 @@ __device__ __forceinline__ bool strip_setup_at(const Geom<T>& g, int seg_rows, i
   return true;
 }
 
+// The calling warp's unit of a whole-grid launch: units count through the
+// strips of one segment before the next segment, so a grid of few strips fills
+// its blocks too.
 template <typename T>
 __device__ __forceinline__ bool strip_setup(const Geom<T>& g, int seg_rows, StripGeom& s) {
-  return strip_setup_at(g, seg_rows, (int)(blockIdx.x * MWPB + (threadIdx.x >> 5)), (int)blockIdx.y, s);
+  const int unit = (int)(blockIdx.x * MWPB + (threadIdx.x >> 5));
+  const int nstrips = (g.nx + MOUT - 1) / MOUT;
+  const int seg = unit / nstrips;
+  if (seg * seg_rows >= g.ny) return false;
+  return strip_setup_at(g, seg_rows, unit - seg * nstrips, seg, s);
 }
 
 // Bottom corners (x, r) and (x+1, r) of one corner row.
@@ -311,14 +318,14 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
 template <typename T> struct MarchStageBlocks { static constexpr int value = sizeof(T) == 4 ? VF_MARCH_STAGE_BLOCKS_F32 : 1; };
 template <typename T> struct MarchFluxBlocks { static constexpr int value = sizeof(T) == 4 ? VF_MARCH_FLUX_BLOCKS_F32 : 1; };
 
-template <typename T, int SEG>
+template <typename T>
 __global__ void __launch_bounds__(MW * MWPB, MarchFluxBlocks<T>::value) k_flux_march(Geom<T> g, Phys<T> p, const T* __restrict__ U,
                                                           const T* __restrict__ B, T* __restrict__ Lout,
-                                                          T* __restrict__ Sout, StepRecord* rec, int parity) {
+                                                          T* __restrict__ Sout, StepRecord* rec, int parity, int seg_rows) {
   if (!rec->active[parity]) return;
   StripGeom s;
   unsigned long long mx = 0ull, my = 0ull;  // CFL maxima as bit patterns (speeds are >= 0)
-  if (strip_setup(g, SEG, s)) flux_march_unit<T, false>(g, p, U, B, Lout, Sout, s, mx, my);
+  if (strip_setup(g, seg_rows, s)) flux_march_unit<T, false>(g, p, U, B, Lout, Sout, s, mx, my);
   block_speed_commit(rec, parity, mx, my);
 }
 
@@ -413,7 +420,8 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
     um2 = mirror_row(un);
   } else {
     um1 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys - 1, xin, cm1, c0, dummy), true);
-    um2 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys - 2, xin, cm2, cm1, dummy), true);
+    if (s.ys == g.gc + 1) um2 = mirror_row(um1);  // one-row segments: the ghost below row gc
+    else um2 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys - 2, xin, cm2, cm1, dummy), true);
   }
   // Ghost row top+1 mirrors row top-2, which leaves the window before it is needed.
   Cell3<T> stash{(T)0, (T)0, (T)0};
@@ -483,12 +491,12 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
   }
 }
 
-template <typename T, int SEG>
+template <typename T>
 __global__ void __launch_bounds__(MW * MWPB, MarchStageBlocks<T>::value) k_stage_march(Geom<T> g, Phys<T> p, const T* __restrict__ U0,
                                                            const T* __restrict__ B, const T* __restrict__ Lin,
                                                            const T* __restrict__ Sin, T* __restrict__ Uo,
-                                                           StepRecord* rec, int parity) {
-  const bool root = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
+                                                           StepRecord* rec, int parity, int seg_rows) {
+  const bool root = blockIdx.x == 0 && threadIdx.x == 0;
   if (!rec->active[parity]) {
     if (root) carry_record(rec, parity);
     return;
@@ -498,7 +506,7 @@ __global__ void __launch_bounds__(MW * MWPB, MarchStageBlocks<T>::value) k_stage
   __syncthreads();
   const double dt = s_dt;
   StripGeom s;
-  if (strip_setup(g, SEG, s)) stage_march_unit<T, false>(g, p, U0, B, Lin, Sin, Uo, s, (T)dt);
+  if (strip_setup(g, seg_rows, s)) stage_march_unit<T, false>(g, p, U0, B, Lin, Sin, Uo, s, (T)dt);
   if (root) advance_record<T>(rec, parity, dt);
 }
 

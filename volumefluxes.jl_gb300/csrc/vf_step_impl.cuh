@@ -17,7 +17,7 @@ static __global__ void k_volume_final_impl(const double* partial, int n, double*
   if (threadIdx.x == 0) *out = red[0];
 }
 
-// Rows per marching segment of the flux and of the stage pass. Shorter
+// Rows per marching segment of the flux and of the stage pass, at most. Shorter
 // segments recompute more halo rows (4 per segment) but give the block
 // scheduler more, smaller units: measured on the Float32 4096^2 step (ms per
 // launch), flux 0.351 / 0.334 / 0.326 / 0.323 / 0.327 at 96 / 64 / 48 / 40 /
@@ -27,6 +27,10 @@ template <typename T> struct MarchSeg {
   static constexpr int flux = 40;
   static constexpr int stage = 24;
 };
+// Warps per SM below which a launch is bound by the latency of one warp's rows
+// (1.2 us a row in the flux pass, 2 us in the stage pass) and not by
+// instruction issue.
+constexpr int kMarchWarpsPerSM = 16;
 
 template <typename T>
 cudaError_t configure_impl() {
@@ -101,10 +105,22 @@ cudaError_t ensemble_max_clusters_impl(int csize, int variant, int* out) {
   return cudaOccupancyMaxActiveClusters(out, k_ensemble<T, 1>, &cfg);
 }
 
+// Segment length of one launch: the shortest that leaves kMarchWarpsPerSM warps
+// on each of the 152 SMs, and at most `longest`. With 40 and 24 rows at every
+// size, a 200x120 grid had 24 and 40 warps on the whole GPU: 51 and 57 us a
+// pass, 5.6 ms for a request of 40 steps instead of 1.7; 1021x511 cells 52 and
+// 62 us a pass, 3.0 ms per 24 steps instead of 1.35 (8 / 16 / 24 / 32 warps:
+// 1.87 / 1.35 / 1.36 / 1.32). From about 2400^2 cells on nothing changes.
 template <typename T>
-dim3 march_grid(const Geom<T>& g, int seg) {
-  const int nstrips = (g.nx + MOUT - 1) / MOUT;
-  return dim3((nstrips + MWPB - 1) / MWPB, (g.ny + seg - 1) / seg);
+int march_seg(const Geom<T>& g, int longest) {
+  const long long nstrips = (g.nx + MOUT - 1) / MOUT, warps = 152LL * kMarchWarpsPerSM;
+  const long long rows = (nstrips * g.ny + warps - 1) / warps;
+  return (int)(rows < longest ? rows : longest);
+}
+template <typename T>
+int march_blocks(const Geom<T>& g, int seg) {
+  const long long units = (long long)((g.nx + MOUT - 1) / MOUT) * ((g.ny + seg - 1) / seg);
+  return (int)((units + MWPB - 1) / MWPB);
 }
 
 // Index of the handle volume Uin is (0 or 1) when the launch can stage its
@@ -133,8 +149,8 @@ cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cud
     }
   }
   if (a.variant == 0) {
-    k_flux_march<T, MarchSeg<T>::flux><<<march_grid(a.g, MarchSeg<T>::flux), MW * MWPB, 0, st>>>(
-        a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity);
+    const int seg = march_seg(a.g, MarchSeg<T>::flux);
+    k_flux_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
     return cudaGetLastError();
   }
   const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
@@ -146,8 +162,9 @@ template <typename T>
 cudaError_t launch_stage_impl(const StepArgs<T>& a, const T* Uin, T* Uout, int parity, cudaStream_t st) {
   const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
   if (a.rk2 && a.variant == 0) {
-    k_stage_march<T, MarchSeg<T>::stage><<<march_grid(a.g, MarchSeg<T>::stage), MW * MWPB, 0, st>>>(
-        a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    const int seg = march_seg(a.g, MarchSeg<T>::stage);
+    k_stage_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity,
+                                                                    seg);
   } else if (a.rk2) {
     if constexpr (sizeof(T) == 8) {
       const int v = tma_volume<T>(a, Uin);
