@@ -423,6 +423,8 @@ int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime
   return push_record(h);
 }
 
+int handle_pull_record(vf_handle* h) { return pull_record(h); }
+
 int handle_enqueue_steps(vf_handle* h, long long first, int n) {
   for (int i = 0; i < n; ++i)
     if (int rc = launch_one_step(h, (int)((first + i) & 1))) return rc;

@@ -3,155 +3,63 @@
 // For a loss of the final state, the reverse sweep carries lambda = dLoss/dU
 // backwards through every step and accumulates dLoss/dB (bottom corners) and
 // dLoss/dCz (friction coefficient). One step is reversed stage by stage, each
-// stage in four kernels that read the recomputed forward data:
+// stage in four launches that read the recomputed forward data:
 //   k_adj_point   the stage's pointwise part in reverse: dry clamp, implicit
-//                 friction (dS/d(w,hu,hv,B_cell,Cz) from dual numbers through
-//                 friction_factor), RK2 average, Euler update; gives
-//                 lambda of L (the stage's time derivative) and the direct
-//                 lambda of the stage input;
-//   k_adj_recon   per cell and direction: lambda of the cell's two face values
-//                 from the central-upwind flux of each adjacent face (local
-//                 Jacobians from dual numbers through cu_face) and from the
-//                 bottom source, then the minmod reconstruction in reverse
-//                 (the subgradient of the branch the forward pass took), split
-//                 into contributions to the cell and its two neighbours;
+//                 friction, RK2 average, Euler update; gives lambda of L (the
+//                 stage's time derivative) and the direct lambda of the stage
+//                 input;
+//   k_adj_face    per face of both directions: lambda of the two face values
+//                 from the lambda of the central-upwind flux through it;
+//   k_adj_recon   per cell of both directions: the bottom source and the minmod
+//                 reconstruction in reverse, split into contributions to the
+//                 cell and its two neighbours;
 //   k_adj_gather  lambda of the stage input per interior cell: the direct part
 //                 plus the neighbour contributions, with the lambda of wall
-//                 ghost cells folded onto the interior cells they mirror;
-//   k_adj_corner  dLoss/dB per corner from the B_cell and face-bottom parts.
-// Dual numbers evaluate the very functions of the forward kernels
-// (vf_math.cuh), so their values -- and every branch -- are the forward
-// pass's; the derivatives follow the branch taken (the subgradient at kinks:
-// minmod switches, dry faces, the dry clamp). Gathers instead of atomics keep
-// the sums in a fixed order: the gradient is deterministic.
+//                 ghost cells folded onto the interior cells they mirror; and,
+//                 in the same launch, dLoss/dB per corner from the B_cell and
+//                 face-bottom parts.
+// The flux and the friction law are reversed by hand, statement by statement:
+// values come from the forward kernels' own expressions (vf_math.cuh), so every
+// branch is the forward pass's, and the derivatives follow the branch taken
+// (the subgradient at kinks: minmod switches, dry faces, the dry clamp). A face
+// costs one forward evaluation and about as many FP64 instructions again for
+// its six derivatives; evaluating it on dual numbers took six forward
+// evaluations per cell and direction, each about twice a plain one (160x128
+// cells, Float64: 113 + 119 us per stage for the two directions, 59 us for the
+// pointwise part with its five dual friction factors, all at ~87% of the FP64
+// pipe). Gathers instead of atomics keep the sums in a fixed order: the
+// gradient is deterministic.
+// A face or cell none of whose incoming lambda is nonzero passes on zeros
+// without evaluating anything: a gauge loss reaches two cells further per stage.
 #pragma once
 #include "vf_kernels.cuh"
 
 namespace vf {
 
-// ---------------------------------------------------------------------------
-// Forward-mode dual numbers on the device.
+// Which operand the forward kernels' max/min returned (also for equal values),
+// so the derivative follows the same operand.
 template <typename T>
-struct Dual {
-  T v, d;
-  __device__ __forceinline__ Dual() : v(0), d(0) {}
-  __device__ __forceinline__ Dual(T x, T dx) : v(x), d(dx) {}
-  template <typename S>
-  __device__ __forceinline__ Dual(S x) : v((T)x), d((T)0) {}  // constants carry no derivative
-};
-
-template <typename T>
-__device__ __forceinline__ Dual<T> operator+(Dual<T> a, Dual<T> b) { return Dual<T>(a.v + b.v, a.d + b.d); }
-template <typename T>
-__device__ __forceinline__ Dual<T> operator-(Dual<T> a, Dual<T> b) { return Dual<T>(a.v - b.v, a.d - b.d); }
-template <typename T>
-__device__ __forceinline__ Dual<T> operator-(Dual<T> a) { return Dual<T>(-a.v, -a.d); }
-// Derivative parts use fused multiply-adds and reciprocals where the value
-// parts keep the forward pass's exact operations: values and branches stay
-// the forward pass's, derivatives change at the rounding level only.
-template <typename T>
-__device__ __forceinline__ Dual<T> operator*(Dual<T> a, Dual<T> b) { return Dual<T>(a.v * b.v, fma(a.d, b.v, a.v * b.d)); }
-template <typename T>
-__device__ __forceinline__ Dual<T> operator/(Dual<T> a, Dual<T> b) {
-  const T q = a.v / b.v;
-  return Dual<T>(q, (a.d - q * b.d) / b.v);
+__device__ __forceinline__ bool picks_second_max(T x, T y) {
+  if constexpr (sizeof(T) == 8) return !(Arith<double>::key(x) > Arith<double>::key(y));
+  return !(x >= y);
 }
 template <typename T>
-__device__ __forceinline__ Dual<T> copysign(Dual<T> a, Dual<T> b) {
-  return Dual<T>(::copysign(a.v, b.v), (T)0);  // used as copysign(1, h): a constant
+__device__ __forceinline__ bool picks_second_min(T x, T y) {
+  if constexpr (sizeof(T) == 8) return !(Arith<double>::key(x) < Arith<double>::key(y));
+  return !(x <= y);
 }
 template <typename T>
-__device__ __forceinline__ Dual<T> fabs(Dual<T> a) {
-  return Dual<T>(::fabs(a.v), ::signbit(a.v) ? -a.d : a.d);
+__device__ __forceinline__ T inverse(T x) {
+  return Arith<T>::inv(Arith<T>::recip(x));
 }
-
 template <typename T>
-struct Arith<Dual<T>> {
-  using A = Arith<T>;
-  using D = Dual<T>;
-  static constexpr bool exact = A::exact;
-  static __device__ __forceinline__ bool lt(D x, D y) { return A::lt(x.v, y.v); }
-  static __device__ __forceinline__ bool gt(D x, D y) { return A::gt(x.v, y.v); }
-  static __device__ __forceinline__ bool gt0(D x) { return A::gt0(x.v); }
-  static __device__ __forceinline__ bool lt0(D x) { return A::lt0(x.v); }
-  static __device__ __forceinline__ bool abs_lt(D x, D k) { return A::abs_lt(x.v, k.v); }
-  static __device__ __forceinline__ bool is_zero(D x) { return A::is_zero(x.v); }
-  // The operand the forward max/min returns, with its derivative.
-  static __device__ __forceinline__ D max(D x, D y) { return picks_second_max(x.v, y.v) ? y : x; }
-  static __device__ __forceinline__ D min(D x, D y) { return picks_second_min(x.v, y.v) ? y : x; }
-  static __device__ __forceinline__ D div(D a, D b) {
-    const T q = A::div(a.v, b.v);
-    return D(q, fma(-q, b.d, a.d) * A::inv(A::recip(b.v)));
-  }
-  static __device__ __forceinline__ D rcp(D b) {
-    const T r = A::rcp(b.v);
-    return D(r, -b.d * r * r);
-  }
-  static __device__ __forceinline__ D sqrt_(D x) {
-    const T r = A::sqrt_(x.v);
-    return D(r, r > (T)0 ? x.d * ((T)0.5 * A::inv(A::recip(r))) : (T)0);
-  }
-  // Quotients over one divisor: values as the forward's div_by, derivatives of a/b.
-  struct Recip {
-    D b;
-    typename A::Recip R;
-  };
-  static __device__ __forceinline__ Recip recip(D b) { return Recip{b, A::recip(b.v)}; }
-  static __device__ __forceinline__ D div_by(const Recip& R, D a) {
-    const T q = A::div_by(R.R, a.v);
-    return D(q, fma(-q, R.b.d, a.d) * A::inv(R.R));
-  }
-  // For equal values the forward max/min may return either operand; these
-  // say which, so the derivative follows the same operand.
-  static __device__ __forceinline__ bool picks_second_max(T x, T y) {
-    if constexpr (sizeof(T) == 8) return !(Arith<double>::key(x) > Arith<double>::key(y));
-    return !(x >= y);
-  }
-  static __device__ __forceinline__ bool picks_second_min(T x, T y) {
-    if constexpr (sizeof(T) == 8) return !(Arith<double>::key(x) < Arith<double>::key(y));
-    return !(x <= y);
-  }
-};
-
-template <>
-__device__ __forceinline__ Dual<double> vcbrt<Dual<double>>(Dual<double> x) {
-  const double r = vcbrt<double>(x.v);
-  return Dual<double>(r, x.v != 0.0 ? x.d * r * Arith<double>::inv(Arith<double>::recip(3.0 * x.v)) : 0.0);
+__device__ __forceinline__ bool all_zero(const T (&v)[3]) {
+  return Arith<T>::is_zero(v[0]) && Arith<T>::is_zero(v[1]) && Arith<T>::is_zero(v[2]);
 }
-template <>
-__device__ __forceinline__ Dual<float> vcbrt<Dual<float>>(Dual<float> x) {
-  const float r = vcbrt<float>(x.v);
-  return Dual<float>(r, x.v != 0.f ? x.d * r / (3.f * x.v) : 0.f);
-}
-
-// The scalars cu_face and friction_factor read, as constants of dual type.
+// d desingularize(h) / dh: |h| / kappa below kappa, where h* = sign(h) (h^2/(2 kappa) + kappa/2).
 template <typename T>
-__device__ __forceinline__ Phys<Dual<T>> dual_phys(const Phys<T>& p) {
-  Phys<Dual<T>> q;
-  q.g = p.g;
-  q.neg_g = p.neg_g;
-  q.rho = p.rho;
-  q.c2 = p.c2;
-  q.cutoff = p.cutoff;
-  q.kappa = p.kappa;
-  q.theta = p.theta;
-  q.inv_dx = p.inv_dx;
-  q.inv_dy = p.inv_dy;
-  q.dx = p.dx;
-  q.dy = p.dy;
-  q.dx_pow2 = p.dx_pow2;
-  q.dy_pow2 = p.dy_pow2;
-  q.dx_exp = p.dx_exp;
-  q.dy_exp = p.dy_exp;
-  q.unit_rho = p.unit_rho;
-  q.Cz = p.Cz;
-  q.near_dry = p.near_dry;
-  q.friction = p.friction;
-  q.n_bottom = p.n_bottom;
-  q.n_point = 0;
-  q.rec_none = p.rec_none;
-  q.any_dynamic = 0;
-  return q;
+__device__ __forceinline__ T desing_slope(T h, T kappa) {
+  return Arith<T>::abs_lt(h, kappa) ? Arith<T>::div(fabs(h), kappa) : (T)1;
 }
 
 // ---------------------------------------------------------------------------
@@ -170,8 +78,9 @@ struct AdjArgs {
   T* lam_direct;        // lambda of Uprev through the pointwise part
   T* lam_base;          // lambda of U^n through the stage-2 average (written by stage 2, read by stage 1)
   T* gBc;               // dLoss/dB_cell per interior cell
-  double* gCz_part;     // one partial sum per block of k_adj_point
-  T* C[2];              // per direction: 9 planes = (to c-1, to c, to c+1) x (w, hu, hv)
+  double* gCz_part;     // one running sum per block of k_adj_point
+  T* C[2];              // per direction: 9 planes = (to c-1, to c, to c+1) x (w, hu, hv); before that, planes
+                        // 0..2 hold lambda of the cell's right face value, 3..5 of its left one
   T* gBf[2];            // per direction: 2 planes (left face bottom, right face bottom) per cell
   T* lam_in;            // gather output: lambda of the stage input
   double* gB;           // dLoss/dB per corner, accumulated
@@ -224,7 +133,7 @@ __global__ void __launch_bounds__(256) k_adj_point(AdjArgs<T> a) {
     T lw = a.lam_out[o], lhu = a.lam_out[g.PS + o], lhv = a.lam_out[2 * g.PS + o];
     T gbc = (T)0;
     if (A::lt(w - Bc, p.cutoff)) {  // dry clamp: (max(w, Bc), 0, 0)
-      if (Arith<Dual<T>>::picks_second_max(w, Bc)) {  // Bc kept
+      if (picks_second_max<T>(w, Bc)) {  // Bc kept
         gbc = gbc + lw;
         lw = (T)0;
       }
@@ -238,21 +147,31 @@ __global__ void __launch_bounds__(256) k_adj_point(AdjArgs<T> a) {
       lhu = lhu / den;
       lhv = lhv / den;
       const T lS = -tdt * lden;
-      const Phys<Dual<T>> dp = dual_phys(p);
-      T grad[5];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        Phys<Dual<T>> pk = dp;
-        if (k == 4) pk.Cz = Dual<T>(p.Cz, (T)1);
-        const Dual<T> dw(q0, k == 0 ? (T)1 : (T)0), dhu(q1, k == 1 ? (T)1 : (T)0), dhv(q2, k == 2 ? (T)1 : (T)0);
-        const Dual<T> dB(Bc, k == 3 ? (T)1 : (T)0);
-        grad[k] = friction_factor<Dual<T>>(pk, dw, dhu, dhv, dB).d;
+      // S = -Cz |u| / den_s(h*) with u = (q1, q2) / h*, h* = desingularize(q0 - Bc)
+      // (src/friction.jl:30-43,62-78), statement by statement in reverse
+      const T h = q0 - Bc;
+      const T hs = desing<T>(h, p.kappa);
+      T u, v;
+      velocities<T>(p, h, hs, q1, q2, u, v);
+      const T speed = A::sqrt_(u * u + v * v);
+      T ds, dds;  // den_s and its derivative
+      if (p.friction == 3) {
+        ds = hs * hs;
+        dds = (T)2 * hs;
+      } else {
+        const T cb = vcbrt<T>(hs);
+        ds = p.friction == 1 ? cb * hs : cb * hs * hs;
+        dds = p.friction == 1 ? cb * (T)(4.0 / 3.0) : cb * hs * (T)(7.0 / 3.0);
       }
-      lq0 = lq0 + lS * grad[0];
-      lq1 = lq1 + lS * grad[1];
-      lq2 = lq2 + lS * grad[2];
-      gbc = gbc + lS * grad[3];
-      gcz = (double)(lS * grad[4]);
+      const T lSd = lS * inverse<T>(ds);
+      gcz = (double)(-lSd * speed);
+      const T lspeed = A::is_zero(speed) ? (T)0 : -lSd * p.Cz * inverse<T>(speed);
+      const T lu = lspeed * u, lv = lspeed * v;
+      const T ihs = inverse<T>(hs);
+      lq1 = lu * ihs;
+      lq2 = lv * ihs;
+      lq0 = (-(lSd * S) * dds - fma(lq1, u, lq2 * v)) * desing_slope<T>(h, p.kappa);
+      gbc = gbc - lq0;
     }
     T lW0 = lw, lW1 = lhu, lW2 = lhv;
     T lb0 = 0, lb1 = 0, lb2 = 0;
@@ -282,7 +201,7 @@ __global__ void __launch_bounds__(256) k_adj_point(AdjArgs<T> a) {
     if (tid < s) red[tid] += red[tid + s];
     __syncthreads();
   }
-  if (tid == 0) a.gCz_part[blockIdx.y * gridDim.x + blockIdx.x] = red[0];
+  if (tid == 0) a.gCz_part[blockIdx.y * gridDim.x + blockIdx.x] += red[0];
 }
 
 // Reverse of minmod_slope (src/reconstruction/linearreconstruction.jl:28-43):
@@ -296,14 +215,14 @@ __device__ __forceinline__ void minmod_slope_rev(T l, T c, T r, T theta, T ls, T
   int pick = -1;
   if (A::gt0(ma) && A::gt0(mb) && A::gt0(mc)) {
     const T m1 = A::min(ma, mb);
-    const int p1 = (m1 == ma && !Arith<Dual<T>>::picks_second_min(ma, mb)) ? 0 : 1;
+    const int p1 = (m1 == ma && !picks_second_min<T>(ma, mb)) ? 0 : 1;
     const T m2 = A::min(m1, mc);
-    pick = (m2 == m1 && !Arith<Dual<T>>::picks_second_min(m1, mc)) ? p1 : 2;
+    pick = (m2 == m1 && !picks_second_min<T>(m1, mc)) ? p1 : 2;
   } else if (A::lt0(ma) && A::lt0(mb) && A::lt0(mc)) {
     const T m1 = A::max(ma, mb);
-    const int p1 = (m1 == ma && !Arith<Dual<T>>::picks_second_max(ma, mb)) ? 0 : 1;
+    const int p1 = (m1 == ma && !picks_second_max<T>(ma, mb)) ? 0 : 1;
     const T m2 = A::max(m1, mc);
-    pick = (m2 == m1 && !Arith<Dual<T>>::picks_second_max(m1, mc)) ? p1 : 2;
+    pick = (m2 == m1 && !picks_second_max<T>(m1, mc)) ? p1 : 2;
   }
   T lf = 0, lb = 0;
   if (pick == 0) lf = theta * ls;
@@ -317,161 +236,239 @@ __device__ __forceinline__ void minmod_slope_rev(T l, T c, T r, T theta, T ls, T
   ll = ll - lb;
 }
 
+// One side of a face as side_flux computes it (n: normal, t: transverse).
+template <typename T>
+struct AdjSide {
+  bool wet;
+  T h, hs, un, ut, f0, fn, ft, c, e1, e2;
+};
+template <typename T, int DIR>
+__device__ __forceinline__ AdjSide<T> adj_side(const Phys<T>& p, const T (&q)[3]) {
+  using A = Arith<T>;
+  AdjSide<T> s{};
+  s.h = q[0];
+  s.wet = A::gt(s.h, p.cutoff);
+  if (!s.wet) return s;
+  s.hs = desing<T>(s.h, p.kappa);
+  T u, v;
+  velocities<T>(p, s.h, s.hs, q[1], q[2], u, v);
+  s.un = DIR == 0 ? u : v;
+  s.ut = DIR == 0 ? v : u;
+  s.f0 = (p.rho * s.h) * s.un;
+  s.fn = s.f0 * s.un + p.c2 * (s.h * s.h);
+  s.ft = s.f0 * s.ut;
+  s.c = A::sqrt_(p.g * s.h);
+  s.e1 = s.un + s.c;
+  s.e2 = s.un - s.c;
+  return s;
+}
+// Adds d(f0, fn, ft, e1, e2)/d(h, hu_n, hu_t) times their lambda to (lh, ln, lt).
+template <typename T>
+__device__ __forceinline__ void adj_side_rev(const Phys<T>& p, const AdjSide<T>& s, T lf0, T lfn, T lft, T le1, T le2,
+                                             T& lh, T& ln, T& lt) {
+  if (!s.wet) return;
+  const T l0 = fma(lft, s.ut, fma(lfn, s.un, lf0));          // of f0, which fn and ft use
+  const T lun = fma(lfn, s.f0, fma(l0, p.rho * s.h, le1 + le2));
+  const T lut = lft * s.f0;
+  const T ihs = inverse<T>(s.hs);
+  const T an = lun * ihs, at = lut * ihs;
+  const T lhs = fma(an, s.un, at * s.ut);
+  T dh = fma(lfn, (T)2 * p.c2 * s.h, l0 * (p.rho * s.un));
+  if (!Arith<T>::is_zero(s.c)) dh = fma(le1 - le2, p.g * ((T)0.5 * inverse<T>(s.c)), dh);
+  lh = lh + fma(-lhs, desing_slope<T>(s.h, p.kappa), dh);
+  ln = ln + an;
+  lt = lt + at;
+}
+
+// cu_face in reverse: lambda of the face values m (minus side) and q (plus side)
+// from lambda of the flux, all in the order (h, hu, hv). With a+, a- the
+// one-sided speeds, d = a+ - a-, N = a+ f(m) - a- f(q):
+// F = N/d + (a+ a-)/d (q - m).
+template <typename T, int DIR>
+__device__ __forceinline__ void face_rev(const Phys<T>& p, const T (&m)[3], const T (&q)[3], const T (&lF)[3],
+                                         T (&lm)[3], T (&lq)[3]) {
+  using A = Arith<T>;
+  constexpr int n = DIR == 0 ? 1 : 2, t = 3 - n;
+  const AdjSide<T> M = adj_side<T, DIR>(p, m), Q = adj_side<T, DIR>(p, q);
+  const bool ap_m = picks_second_max<T>(Q.e1, M.e1), am_m = picks_second_min<T>(Q.e2, M.e2);
+  const T ap1 = ap_m ? M.e1 : Q.e1, am1 = am_m ? M.e2 : Q.e2;
+  const bool ap_0 = picks_second_max<T>(ap1, (T)0), am_0 = picks_second_min<T>(am1, (T)0);
+  const T ap = ap_0 ? (T)0 : ap1, am = am_0 ? (T)0 : am1;
+  const T d = ap - am;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) lm[k] = lq[k] = (T)0;
+  if (A::abs_lt(d, p.kappa)) return;
+  const T id = inverse<T>(d);
+  const T l0 = lF[0] * id, ln = lF[n] * id, lt = lF[t] * id;  // of N
+  const T N0 = fma(ap, M.f0, -(am * Q.f0)), Nn = fma(ap, M.fn, -(am * Q.fn)), Nt = fma(ap, M.ft, -(am * Q.ft));
+  const T qa = ap * am * id;
+  // of the product a+ a-, and of d through both quotients
+  const T lp = fma(l0, q[0] - m[0], fma(ln, q[n] - m[n], lt * (q[t] - m[t])));
+  const T ld = -(fma(l0, N0, fma(ln, Nn, lt * Nt)) * id + lp * qa);
+  const T lap = fma(l0, M.f0, fma(ln, M.fn, fma(lt, M.ft, fma(lp, am, ld))));
+  const T lam = fma(-l0, Q.f0, fma(-ln, Q.fn, fma(-lt, Q.ft, fma(lp, ap, -ld))));
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    lm[k] = -(lF[k] * qa);
+    lq[k] = lF[k] * qa;
+  }
+  const T z = (T)0;
+  adj_side_rev<T>(p, M, ap * l0, ap * ln, ap * lt, !ap_0 && ap_m ? lap : z, !am_0 && am_m ? lam : z, lm[0], lm[n], lm[t]);
+  adj_side_rev<T>(p, Q, -(am * l0), -(am * ln), -(am * lt), !ap_0 && !ap_m ? lap : z, !am_0 && !am_m ? lam : z, lq[0],
+                  lq[n], lq[t]);
+}
+
+// Access along DIR at (al + s, ac): al along, ac across.
+template <typename T, int DIR>
+struct AdjLine {
+  const AdjArgs<T>& a;
+  int al, ac, n_al;
+  __device__ __forceinline__ int x(int s) const { return DIR == 0 ? al + s : ac; }
+  __device__ __forceinline__ int y(int s) const { return DIR == 0 ? ac : al + s; }
+  __device__ __forceinline__ void state(int s, T (&u)[3]) const {
+    const Geom<T>& g = a.g;
+    const bool in = x(s) >= 0 && y(s) >= 0 && x(s) < g.N1 && y(s) < g.N2;
+    const long long o = sidx(g, x(s), y(s));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) u[k] = in ? a.Uprev[k * g.PS + o] : (T)0;
+  }
+  __device__ __forceinline__ void lamL(int s, T (&l)[3]) const {  // of L at an interior cell, else 0
+    const Geom<T>& g = a.g;
+    const bool in = al + s >= g.gc && al + s < g.gc + n_al;
+    const long long o = sidx(g, x(s), y(s));
+#pragma unroll
+    for (int k = 0; k < 3; ++k) l[k] = in ? a.lamL[k * g.PS + o] : (T)0;
+  }
+  // bottom of the face left of the cell at offset s
+  __device__ __forceinline__ T bface(int s) const {
+    if (a.g.bottom_const) return a.g.bconst;
+    const long long b = (long long)y(s) * a.g.PB + x(s) + XOFF;
+    return halve<T>(a.B[b] + (DIR == 0 ? a.B[b + a.g.PB] : a.B[b + 1]));
+  }
+  __device__ __forceinline__ T bcell(int s) const { return cell_bottom(a.g, a.B, x(s), y(s)); }
+  // face values of the cell at offset s, as the forward pass reconstructs them
+  __device__ __forceinline__ void faces(int s, const T (&l)[3], const T (&c)[3], const T (&r)[3], T (&L)[3],
+                                        T (&R)[3]) const {
+    if (a.p.rec_none) no_reconstruction<T>(c, bcell(s), L, R);
+    else reconstruct_cell<T>(a.p, l, c, r, bface(s), bface(s + 1), L, R);
+  }
+};
+
+// Faces along DIR: face f lies between the cells gc-1+f and gc+f, f = 0..n.
+template <typename T, int DIR>
+__device__ __forceinline__ void adj_face(const AdjArgs<T>& a, int ix, int iy) {
+  const Geom<T>& g = a.g;
+  const int f = DIR == 0 ? ix : iy, n_al = DIR == 0 ? g.nx : g.ny;
+  if (ix >= g.nx + (DIR == 0) || iy >= g.ny + (DIR == 1)) return;
+  const AdjLine<T, DIR> c{a, g.gc - 1 + f, g.gc + (DIR == 0 ? iy : ix), n_al};
+  T lmc[3], lpc[3], lF[3], lm[3] = {0, 0, 0}, lq[3] = {0, 0, 0};
+  c.lamL(0, lmc);
+  c.lamL(1, lpc);
+  const T inv = DIR == 0 ? a.p.inv_dx : a.p.inv_dy;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) lF[k] = inv * (lpc[k] - lmc[k]);
+  if (!all_zero(lF)) {
+    T u0[3], u1[3], u2[3], u3[3], t[3], m[3], q[3];
+    c.state(-1, u0);
+    c.state(0, u1);
+    c.state(1, u2);
+    c.state(2, u3);
+    c.faces(0, u0, u1, u2, t, m);
+    c.faces(1, u1, u2, u3, q, t);
+    face_rev<T, DIR>(a.p, m, q, lF, lm, lq);
+  }
+  const long long om = sidx(g, c.x(0), c.y(0)), oq = sidx(g, c.x(1), c.y(1));
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    a.C[DIR][k * g.PS + om] = lm[k];
+    a.C[DIR][(3 + k) * g.PS + oq] = lq[k];
+  }
+}
+// blockIdx.z: direction; threadIdx.x runs along x in both, so loads coalesce.
+template <typename T>
+__global__ void __launch_bounds__(128) k_adj_face(AdjArgs<T> a) {
+  const int ix = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y * blockDim.y + threadIdx.y;
+  if (blockIdx.z == 0) adj_face<T, 0>(a, ix, iy);
+  else adj_face<T, 1>(a, ix, iy);
+}
+
 // Per cell of the reconstruction range along DIR (the first ghost layer
 // included, src/reconstruction/linearreconstruction.jl:60-68), interior across.
 template <typename T, int DIR>
-__global__ void __launch_bounds__(128) k_adj_recon(AdjArgs<T> a) {
+__device__ __forceinline__ void adj_recon(const AdjArgs<T>& a, int ix, int iy) {
   using A = Arith<T>;
   const Geom<T>& g = a.g;
   const Phys<T>& p = a.p;
-  // along: cells gc-1 .. gc+n; across: interior
   const int n_al = DIR == 0 ? g.nx : g.ny;
-  const int n_ac = DIR == 0 ? g.ny : g.nx;
-  const int al = g.gc - 1 + blockIdx.x * blockDim.x + threadIdx.x;
-  const int ac = g.gc + blockIdx.y * blockDim.y + threadIdx.y;
-  if (al > g.gc + n_al || ac >= g.gc + n_ac) return;
-  auto X = [&](int s) { return DIR == 0 ? al + s : ac; };
-  auto Y = [&](int s) { return DIR == 0 ? ac : al + s; };
-  auto ld = [&](int s, int k) -> T {
-    const int xx = X(s), yy = Y(s);
-    if (xx < 0 || yy < 0 || xx >= g.N1 || yy >= g.N2) return (T)0;
-    return a.Uprev[k * g.PS + sidx(g, xx, yy)];
-  };
-  auto lamL = [&](int s, int k) -> T {  // lambda of L at an interior cell, else 0
-    const int at = al + s;
-    if (at < g.gc || at >= g.gc + n_al) return (T)0;
-    return a.lamL[k * g.PS + sidx(g, X(s), Y(s))];
-  };
-  // bottom faces of cell at offset s along DIR
-  auto bface = [&](int s, int right) -> T {
-    if (g.bottom_const) return g.bconst;
-    const int xx = X(s), yy = Y(s);
-    const long long b = (long long)yy * g.PB + xx + XOFF;
-    if (DIR == 0) {
-      return right ? (T)0.5 * (a.B[b + 1] + a.B[b + 1 + g.PB]) : (T)0.5 * (a.B[b] + a.B[b + g.PB]);
-    }
-    return right ? (T)0.5 * (a.B[b + g.PB] + a.B[b + g.PB + 1]) : (T)0.5 * (a.B[b] + a.B[b + 1]);
-  };
-  // B_cell of the cell at offset s along DIR, in the forward kernels' order
-  // (NoReconstruction's face depth is w - B_cell, src/reconstruction/noreconstruction.jl:30-46)
-  auto bcell = [&](int s) -> T {
-    if (g.bottom_const) return g.bconst;
-    const long long b = (long long)Y(s) * g.PB + X(s) + XOFF;
-    return (T)0.25 * (((a.B[b] + a.B[b + 1]) + a.B[b + g.PB]) + a.B[b + g.PB + 1]);
-  };
-  const T inv = DIR == 0 ? p.inv_dx : p.inv_dy;
-  // Stencil values at offsets -2..+2 (only what is used is read).
-  T u[5][3];
+  if (ix >= g.nx + 2 * (DIR == 0) || iy >= g.ny + 2 * (DIR == 1)) return;
+  const AdjLine<T, DIR> c{a, g.gc - 1 + (DIR == 0 ? ix : iy), g.gc + (DIR == 0 ? iy : ix), n_al};
+  const bool face_r = c.al <= g.gc + n_al - 1;  // face c+1/2 is used
+  const bool face_l = c.al >= g.gc;             // face c-1/2 is used
+  const long long o = sidx(g, c.x(0), c.y(0));
+  T lR[3], lL[3], lam[3];
 #pragma unroll
-  for (int s = 0; s < 5; ++s)
-#pragma unroll
-    for (int k = 0; k < 3; ++k) u[s][k] = ld(s - 2, k);
-  const bool face_r = al <= g.gc + n_al - 1;  // face c+1/2 is used
-  const bool face_l = al >= g.gc;             // face c-1/2 is used
-  // reconstruction of cells c-1, c, c+1 (forward)
-  T Lc[3], Rc[3], Rm[3], Lp[3];
-  const T Blc = bface(0, 0), Brc = bface(0, 1);
-  if (p.rec_none) {
-    no_reconstruction<T>(u[2], bcell(0), Lc, Rc);
-    T tmp[3];
-    if (face_l) no_reconstruction<T>(u[1], bcell(-1), tmp, Rm);
-    if (face_r) no_reconstruction<T>(u[3], bcell(1), Lp, tmp);
-  } else {
-    reconstruct_cell<T>(p, u[1], u[2], u[3], Blc, Brc, Lc, Rc);
-    if (face_l) {
-      T Lm[3];
-      reconstruct_cell<T>(p, u[0], u[1], u[2], bface(-1, 0), bface(-1, 1), Lm, Rm);
-    }
-    if (face_r) {
-      T Rp[3];
-      reconstruct_cell<T>(p, u[2], u[3], u[4], bface(1, 0), bface(1, 1), Lp, Rp);
-    }
+  for (int k = 0; k < 3; ++k) {
+    lR[k] = face_r ? a.C[DIR][k * g.PS + o] : (T)0;
+    lL[k] = face_l ? a.C[DIR][(3 + k) * g.PS + o] : (T)0;
   }
-  T lR[3] = {0, 0, 0}, lL[3] = {0, 0, 0};
-  const Phys<Dual<T>> dp = dual_phys(p);
-  if (face_r) {  // face between c and c+1: c is the minus side
-    T lF[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) lF[k] = inv * (lamL(1, k) - lamL(0, k));
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      Dual<T> m[3], q[3], F[3], sp;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        m[k] = Dual<T>(Rc[k], j == k ? (T)1 : (T)0);
-        q[k] = Dual<T>(Lp[k], (T)0);
-      }
-      cu_face<Dual<T>, DIR, false>(dp, m[0], m[1], m[2], q[0], q[1], q[2], F[0], F[1], F[2], sp);
-      lR[j] = (lF[0] * F[0].d + lF[1] * F[1].d) + lF[2] * F[2].d;
-    }
-  }
-  if (face_l) {  // face between c-1 and c: c is the plus side
-    T lF[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) lF[k] = inv * (lamL(0, k) - lamL(-1, k));
-#pragma unroll
-    for (int j = 0; j < 3; ++j) {
-      Dual<T> m[3], q[3], F[3], sp;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) {
-        m[k] = Dual<T>(Rm[k], (T)0);
-        q[k] = Dual<T>(Lc[k], j == k ? (T)1 : (T)0);
-      }
-      cu_face<Dual<T>, DIR, false>(dp, m[0], m[1], m[2], q[0], q[1], q[2], F[0], F[1], F[2], sp);
-      lL[j] = (lF[0] * F[0].d + lF[1] * F[1].d) + lF[2] * F[2].d;
-    }
-  }
-  // bottom source of interior cells (src/sourceterms/source_term_bottom.jl:24-41)
+  c.lamL(0, lam);
   T gBl = 0, gBr = 0;
-  if (face_l && face_r && p.n_bottom > 0) {
-    const int kk = DIR == 0 ? 1 : 2;
-    const T lk = lamL(0, kk) * (T)p.n_bottom;
-    const T slope = slope_over<T>(Brc - Blc, DIR == 0 ? p.dx : p.dy, inv, DIR == 0 ? p.dx_pow2 : p.dy_pow2);
-    const T hmean = (Rc[0] + Lc[0]) * (T)0.5;
-    lR[0] = lR[0] + lk * p.neg_g * slope * (T)0.5;
-    lL[0] = lL[0] + lk * p.neg_g * slope * (T)0.5;
-    const T ldb = lk * p.neg_g * hmean * inv;  // d(dB/Δ)/d(dB) = 1/Δ
-    gBr = gBr + ldb;
-    gBl = gBl - ldb;
-  }
-  // reconstruction of cell c in reverse
   T lu[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};  // [neighbour -1, 0, +1][component]
-  if (p.rec_none) {
-    // L = R = (w - B_cell, hu, hv): the cell takes both faces' lambda, and
-    // d/dB_cell = -(lambda_L.h + lambda_R.h) goes to the corners a quarter
-    // each, i.e. half to each face bottom of this direction (whose corners
-    // are the cell's, a half each)
+  if (!(all_zero(lR) && all_zero(lL) && all_zero(lam))) {
+    const T inv = DIR == 0 ? p.inv_dx : p.inv_dy;
+    const T Blc = c.bface(0), Brc = c.bface(1);
+    T ul[3], uc[3], ur[3], Lc[3], Rc[3];
+    c.state(-1, ul);
+    c.state(0, uc);
+    c.state(1, ur);
+    // bottom source of interior cells (src/sourceterms/source_term_bottom.jl:24-41)
+    if (face_l && face_r && p.n_bottom > 0) {
+      c.faces(0, ul, uc, ur, Lc, Rc);
+      const T lk = lam[DIR == 0 ? 1 : 2] * (T)p.n_bottom;
+      const T slope = slope_over<T>(Brc - Blc, DIR == 0 ? p.dx : p.dy, inv, DIR == 0 ? p.dx_pow2 : p.dy_pow2);
+      const T hmean = (Rc[0] + Lc[0]) * (T)0.5;
+      lR[0] = lR[0] + lk * p.neg_g * slope * (T)0.5;
+      lL[0] = lL[0] + lk * p.neg_g * slope * (T)0.5;
+      const T ldb = lk * p.neg_g * hmean * inv;  // d(dB/Δ)/d(dB) = 1/Δ
+      gBr = gBr + ldb;
+      gBl = gBl - ldb;
+    }
+    // reconstruction of cell c in reverse
+    if (p.rec_none) {
+      // L = R = (w - B_cell, hu, hv): the cell takes both faces' lambda, and
+      // d/dB_cell = -(lambda_L.h + lambda_R.h) goes to the corners a quarter
+      // each, i.e. half to each face bottom of this direction (whose corners
+      // are the cell's, a half each)
 #pragma unroll
-    for (int k = 0; k < 3; ++k) lu[1][k] = lL[k] + lR[k];
-    const T dBc = (T)0 - (lL[0] + lR[0]);
-    gBl = gBl + (T)0.5 * dBc;
-    gBr = gBr + (T)0.5 * dBc;
-  }
-#pragma unroll
-  for (int k = 1; k < 3 && !p.rec_none; ++k) {  // hu, hv: L = c - s/2, R = c + s/2
-    lu[1][k] = lu[1][k] + lL[k] + lR[k];
-    const T ls = (T)0.5 * (lR[k] - lL[k]);
-    minmod_slope_rev<T>(u[1][k], u[2][k], u[3][k], p.theta, ls, lu[0][k], lu[1][k], lu[2][k]);
-  }
-  if (!p.rec_none) {  // w with the bottom-limited slope
-    const T w = u[2][0];
-    const T s0 = minmod_slope<T>(u[1][0], u[2][0], u[3][0], p.theta);
-    // L0 = (w - s/2) - Bl, R0 = (w + s/2) - Br
-    lu[1][0] = lu[1][0] + lL[0] + lR[0];
-    gBl = gBl - lL[0];
-    gBr = gBr - lR[0];
-    const T ls = (T)0.5 * (lR[0] - lL[0]);
-    if (A::lt(w - (T)0.5 * s0, Blc)) {          // s = 2(w - Bl)
-      lu[1][0] = lu[1][0] + (T)2 * ls;
-      gBl = gBl - (T)2 * ls;
-    } else if (A::lt(w + (T)0.5 * s0, Brc)) {   // s = 2(Br - w)
-      lu[1][0] = lu[1][0] - (T)2 * ls;
-      gBr = gBr + (T)2 * ls;
+      for (int k = 0; k < 3; ++k) lu[1][k] = lL[k] + lR[k];
+      const T dBc = (T)0 - (lL[0] + lR[0]);
+      gBl = gBl + (T)0.5 * dBc;
+      gBr = gBr + (T)0.5 * dBc;
     } else {
-      minmod_slope_rev<T>(u[1][0], u[2][0], u[3][0], p.theta, ls, lu[0][0], lu[1][0], lu[2][0]);
+#pragma unroll
+      for (int k = 1; k < 3; ++k) {  // hu, hv: L = c - s/2, R = c + s/2
+        lu[1][k] = lL[k] + lR[k];
+        const T ls = (T)0.5 * (lR[k] - lL[k]);
+        minmod_slope_rev<T>(ul[k], uc[k], ur[k], p.theta, ls, lu[0][k], lu[1][k], lu[2][k]);
+      }
+      // w with the bottom-limited slope: L0 = (w - s/2) - Bl, R0 = (w + s/2) - Br
+      const T w = uc[0];
+      const T s0 = minmod_slope<T>(ul[0], uc[0], ur[0], p.theta);
+      lu[1][0] = lL[0] + lR[0];
+      gBl = gBl - lL[0];
+      gBr = gBr - lR[0];
+      const T ls = (T)0.5 * (lR[0] - lL[0]);
+      if (A::lt(w - (T)0.5 * s0, Blc)) {          // s = 2(w - Bl)
+        lu[1][0] = lu[1][0] + (T)2 * ls;
+        gBl = gBl - (T)2 * ls;
+      } else if (A::lt(w + (T)0.5 * s0, Brc)) {   // s = 2(Br - w)
+        lu[1][0] = lu[1][0] - (T)2 * ls;
+        gBr = gBr + (T)2 * ls;
+      } else {
+        minmod_slope_rev<T>(ul[0], uc[0], ur[0], p.theta, ls, lu[0][0], lu[1][0], lu[2][0]);
+      }
     }
   }
-  const long long o = sidx(g, X(0), Y(0));
   T* C = a.C[DIR];
 #pragma unroll
   for (int nb = 0; nb < 3; ++nb)
@@ -480,15 +477,19 @@ __global__ void __launch_bounds__(128) k_adj_recon(AdjArgs<T> a) {
   a.gBf[DIR][o] = gBl;
   a.gBf[DIR][g.PS + o] = gBr;
 }
+template <typename T>
+__global__ void __launch_bounds__(128) k_adj_recon(AdjArgs<T> a) {
+  const int ix = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y * blockDim.y + threadIdx.y;
+  if (blockIdx.z == 0) adj_recon<T, 0>(a, ix, iy);
+  else adj_recon<T, 1>(a, ix, iy);
+}
 
 // lambda of the stage input per interior cell: direct part + neighbour
 // contributions, with the lambda of wall ghost cells folded onto the interior
 // cells they mirror (src/bc.jl:81-110; x ghosts negate hu, y ghosts hv).
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_gather(AdjArgs<T> a) {
+__device__ __forceinline__ void adj_gather(const AdjArgs<T>& a, int x, int y) {
   const Geom<T>& g = a.g;
-  const int x = g.gc + blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = g.gc + blockIdx.y * blockDim.y + threadIdx.y;
   if (x >= g.gc + g.nx || y >= g.gc + g.ny) return;
   // contributions landing on cell (xx, yy) from the reconstructions along DIR
   auto land = [&](int dir, int xx, int yy, int k) -> T {
@@ -548,10 +549,8 @@ __global__ void __launch_bounds__(256) k_adj_gather(AdjArgs<T> a) {
 
 // dLoss/dB per corner (I, J) of the (N1+1) x (N2+1) corner grid.
 template <typename T>
-__global__ void __launch_bounds__(256) k_adj_corner(AdjArgs<T> a) {
+__device__ __forceinline__ void adj_corner(const AdjArgs<T>& a, int I, int J) {
   const Geom<T>& g = a.g;
-  const int I = blockIdx.x * blockDim.x + threadIdx.x;
-  const int J = blockIdx.y * blockDim.y + threadIdx.y;
   if (I > g.N1 || J > g.N2) return;
   auto cellv = [&](const T* arr, int cx, int cy) -> double {
     if (cx < 0 || cy < 0 || cx >= g.N1 || cy >= g.N2) return 0.0;
@@ -580,6 +579,27 @@ __global__ void __launch_bounds__(256) k_adj_corner(AdjArgs<T> a) {
   a.gB[(long long)J * (g.N1 + 1) + I] += s;
 }
 
+// blockIdx.z 0: lambda of the stage input; 1: dLoss/dB. Both read what the
+// earlier launches of the stage wrote and neither what the other writes.
+template <typename T>
+__global__ void __launch_bounds__(256) k_adj_gather(AdjArgs<T> a) {
+  const int ix = blockIdx.x * blockDim.x + threadIdx.x, iy = blockIdx.y * blockDim.y + threadIdx.y;
+  if (blockIdx.z == 0) adj_gather<T>(a, a.g.gc + ix, a.g.gc + iy);
+  else adj_corner<T>(a, ix, iy);
+}
+
+// The step record of a reversed or recomputed step: dt forced, start time t.
+static __global__ void k_adj_record(StepRecord* rec, double dt, double t) {
+  StepRecord r = {};
+  r.active[0] = 1;
+  r.t[0] = t;
+  r.explicit_mode = 1;
+  r.force_dt = 1;
+  r.forced_dt = dt;
+  r.wait_fault = rec->wait_fault;  // kept until the host reads the record
+  *rec = r;
+}
+
 // lambda of the final state from the gauge loss sum_g (w[g] - target[g])^2,
 // and the loss, in gauge order (one thread).
 template <typename T>
@@ -596,12 +616,18 @@ __global__ void k_adj_seed(Geom<T> g, const T* U, T* lam, const int* gi, const i
   *loss = L;
 }
 
-// Sum of the per-block dLoss/dCz partials into *acc, in block order (one thread).
+// Sum of the per-block dLoss/dCz sums into *acc, in a fixed order (one block).
 static __global__ void k_adj_sum(const double* part, int n, double* acc) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  __shared__ double red[256];
   double s = 0.0;
-  for (int i = 0; i < n; ++i) s += part[i];
-  *acc += s;
+  for (int i = threadIdx.x; i < n; i += 256) s += part[i];
+  red[threadIdx.x] = s;
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) *acc = red[0];
 }
 
 }  // namespace vf

@@ -39,14 +39,15 @@ struct vf_adjoint {
   void* C[2] = {nullptr, nullptr};    // 9 planes each
   void* gBf[2] = {nullptr, nullptr};  // 2 planes each
   double* gB = nullptr;    // (N1+1) x (N2+1)
-  double* gCz_part = nullptr;
+  double* gCz_part = nullptr;  // running sums, one per block of the pointwise kernel
+  int gCz_blocks = 0;
   double* gCz = nullptr;
   double* loss = nullptr;
   int* gauges = nullptr;
   double* target = nullptr;
   int gauge_cap = 0;
   vf::StepRecord* rec = nullptr;
-  vf::StepRecord rec_h;
+  double* dts_d = nullptr;  // dt of every step of the forward pass
   std::vector<double> dts;
   std::vector<double> ts;  // start time of every step of the forward pass (time-dependent sources)
   bool have_forward = false;
@@ -75,7 +76,7 @@ void free_all(vf_adjoint* a) {
   cudaStream_t st = a->h ? a->h->stream : nullptr;
   void* ps[] = {a->init, a->ckpt, a->seg, a->U1, a->L0, a->L1, a->S0, a->S1, a->lam, a->lamU1, a->lamL,
                 a->lam_direct, a->lam_base, a->gBc, a->C[0], a->C[1], a->gBf[0], a->gBf[1], a->gB,
-                a->gCz_part, a->gCz, a->loss, a->gauges, a->target, a->rec};
+                a->gCz_part, a->gCz, a->loss, a->gauges, a->target, a->rec, a->dts_d};
   for (void* p : ps)
     if (p) cudaFreeAsync(p, st);
   if (st) cudaStreamSynchronize(st);
@@ -99,15 +100,7 @@ template <>
 vf::StepArgs<float>& args_of<float>(vf_handle* h) { return h->af; }
 
 int set_dt(vf_adjoint* a, double dt, double t) {
-  std::memset(&a->rec_h, 0, sizeof(a->rec_h));
-  a->rec_h.active[0] = 1;
-  a->rec_h.t[0] = t;
-  a->rec_h.explicit_mode = 1;
-  a->rec_h.force_dt = 1;
-  a->rec_h.forced_dt = dt;
-  VF_ACK(a, cudaMemcpyAsync(a->rec, &a->rec_h, sizeof(vf::StepRecord), cudaMemcpyHostToDevice, a->h->stream));
-  // the record is pageable host memory: let the copy finish before it changes
-  VF_ACK(a, cudaStreamSynchronize(a->h->stream));
+  VF_ACK(a, vf::launch_adj_record(a->rec, dt, t, a->h->stream));
   return VF_OK;
 }
 
@@ -149,18 +142,15 @@ vf::AdjArgs<T> adj_args(vf_adjoint* a, double dt) {
   return x;
 }
 
-// One stage in reverse: pointwise part, both reconstructions, gather, corners.
+// One stage in reverse: pointwise part, faces, reconstructions, gather with corners.
 template <typename T>
 int reverse_stage(vf_adjoint* a, vf::AdjArgs<T> x) {
   cudaStream_t st = a->h->stream;
-  int nb = 0;
-  VF_ACK(a, vf::launch_adj_point(x, &nb, st));
-  VF_ACK(a, vf::launch_adj_sum(a->gCz_part, nb, a->gCz, st));
-  VF_ACK(a, vf::launch_adj_recon(x, 0, st));
-  VF_ACK(a, vf::launch_adj_recon(x, 1, st));
+  VF_ACK(a, vf::launch_adj_point(x, &a->gCz_blocks, st));
+  VF_ACK(a, vf::launch_adj_face(x, st));
+  VF_ACK(a, vf::launch_adj_recon(x, st));
   VF_ACK(a, vf::launch_adj_gather(x, st));
-  VF_ACK(a, vf::launch_adj_corner(x, st));
-  a->h->launches += 6;
+  a->h->launches += 4;
   return VF_OK;
 }
 
@@ -242,7 +232,7 @@ int backward_impl(vf_adjoint* a, const int32_t* gi, const int32_t* gj, const dou
   VF_ACK(a, cudaMemcpyAsync(a->target, target, sizeof(double) * (size_t)n_g, cudaMemcpyHostToDevice, st));
   VF_ACK(a, cudaMemsetAsync(a->lam, 0, a->state_bytes, st));
   VF_ACK(a, cudaMemsetAsync(a->gB, 0, sizeof(double) * (size_t)(g.N1 + 1) * (g.N2 + 1), st));
-  VF_ACK(a, cudaMemsetAsync(a->gCz, 0, sizeof(double), st));
+  VF_ACK(a, cudaMemsetAsync(a->gCz_part, 0, sizeof(double) * (size_t)((g.nx + 31) / 32) * ((g.ny + 7) / 8), st));
   VF_ACK(a, vf::launch_adj_seed(g, static_cast<const T*>(h->U[0]), static_cast<T*>(a->lam), a->gauges,
                                 a->gauges + n_g, a->target, n_g, a->loss, st));
   VF_ACK(a, cudaStreamSynchronize(st));  // the host vectors above go out of scope
@@ -259,6 +249,7 @@ int backward_impl(vf_adjoint* a, const int32_t* gi, const int32_t* gj, const dou
       if (int rc = reverse_step<T>(a, off(a->seg, (size_t)(n - start) * a->state_bytes), a->dts[n], a->ts[n]))
         return rc;
   }
+  VF_ACK(a, vf::launch_adj_sum(a->gCz_part, a->gCz_blocks, a->gCz, st));
   double gcz = 0, loss = 0;
   VF_ACK(a, cudaMemcpyAsync(&gcz, a->gCz, sizeof(double), cudaMemcpyDeviceToHost, st));
   VF_ACK(a, cudaMemcpyAsync(&loss, a->loss, sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -268,6 +259,64 @@ int backward_impl(vf_adjoint* a, const int32_t* gi, const int32_t* gj, const dou
   VF_ACK(a, cudaStreamSynchronize(st));
   if (grad_Cz) *grad_Cz = gcz;
   if (loss_out) *loss_out = loss;
+  return VF_OK;
+}
+
+// ---- forward pass -----------------------------------------------------------
+int restart(vf_adjoint* a) {
+  VF_ACK(a, cudaMemcpyAsync(a->h->U[0], a->init, a->state_bytes, cudaMemcpyDeviceToDevice, a->h->stream));
+  return VF_OK;
+}
+int checkpoint(vf_adjoint* a, int n, const void* U) {
+  if (n % a->K == 0)
+    VF_ACK(a, cudaMemcpyAsync(off(a->ckpt, (size_t)(n / a->K) * a->state_bytes), U, a->state_bytes,
+                              cudaMemcpyDeviceToDevice, a->h->stream));
+  return VF_OK;
+}
+
+// Every step with its CFL dt, the clock on the device and one synchronisation
+// at the end (one per step cost 9 round trips of ~25 us on a 9-step run).
+int forward_cfl(vf_adjoint* a) {
+  vf_handle* h = a->h;
+  if (int rc = restart(a)) return rc;
+  if (int rc = vf::handle_begin_loop(h, 0.0, INFINITY, 0, -1.0)) return afail(a, rc, "forward step: " + h->err);
+  for (int n = 0; n < a->n_steps; ++n) {
+    if (int rc = checkpoint(a, n, h->U[n & 1])) return rc;
+    if (int rc = vf::handle_enqueue_steps(h, n, 1)) return afail(a, rc, "forward step: " + h->err);
+    VF_ACK(a, cudaMemcpyAsync(a->dts_d + n, &h->rec->last_dt, sizeof(double), cudaMemcpyDeviceToDevice, h->stream));
+  }
+  VF_ACK(a, cudaMemcpyAsync(a->dts.data(), a->dts_d, sizeof(double) * a->n_steps, cudaMemcpyDeviceToHost, h->stream));
+  if (int rc = vf::handle_pull_record(h)) return afail(a, rc, "forward step: " + h->err);
+  if (a->n_steps & 1) std::swap(h->U[0], h->U[1]);
+  return VF_OK;
+}
+
+// Every step with the dt of a->dts.
+int forward_frozen(vf_adjoint* a) {
+  vf_handle* h = a->h;
+  if (int rc = restart(a)) return rc;
+  VF_ACK(a, cudaMemsetAsync(h->rec, 0, sizeof(vf::StepRecord), h->stream));
+  double t = 0.0;
+  for (int n = 0; n < a->n_steps; ++n) {
+    if (int rc = checkpoint(a, n, h->U[0])) return rc;
+    VF_ACK(a, vf::launch_adj_record(h->rec, a->dts[n], t, h->stream));
+    if (int rc = vf::handle_enqueue_steps(h, 0, 1)) return afail(a, rc, "forward step: " + h->err);
+    std::swap(h->U[0], h->U[1]);
+    t += a->dts[n];
+  }
+  if (int rc = vf::handle_pull_record(h)) return afail(a, rc, "forward step: " + h->err);
+  return VF_OK;
+}
+
+int forward_stepwise(vf_adjoint* a) {
+  vf_handle* h = a->h;
+  if (int rc = restart(a)) return rc;
+  double t = 0.0;
+  for (int n = 0; n < a->n_steps; ++n) {
+    if (int rc = checkpoint(a, n, h->U[0])) return rc;
+    if (int rc = vf_step(h, INFINITY, t, &a->dts[n])) return afail(a, rc, "forward step: " + h->err);
+    t += a->dts[n];
+  }
   return VF_OK;
 }
 
@@ -320,7 +369,8 @@ int vf_adjoint_create(vf_handle* h, int32_t n_steps, int32_t checkpoint_every, v
                                                                  ((h->cfg.ny + 7) / 8)) &&
             alloc(a, reinterpret_cast<void**>(&a->gCz), sizeof(double)) &&
             alloc(a, reinterpret_cast<void**>(&a->loss), sizeof(double)) &&
-            alloc(a, reinterpret_cast<void**>(&a->rec), sizeof(vf::StepRecord));
+            alloc(a, reinterpret_cast<void**>(&a->rec), sizeof(vf::StepRecord)) &&
+            alloc(a, reinterpret_cast<void**>(&a->dts_d), sizeof(double) * (size_t)n_steps);
   ok = ok && cudaMemcpyAsync(a->init, h->U[0], a->state_bytes, cudaMemcpyDeviceToDevice, h->stream) == cudaSuccess;
   ok = ok && cudaStreamSynchronize(h->stream) == cudaSuccess;
   if (!ok) {
@@ -337,26 +387,31 @@ int vf_adjoint_forward(vf_adjoint* a, const double* frozen_dts, double* dts_out)
   if (!a) return afail(nullptr, VF_EINVAL, "NULL adjoint");
   vf_handle* h = a->h;
   VF_ACK(a, cudaSetDevice(h->device));
-  VF_ACK(a, cudaMemcpyAsync(h->U[0], a->init, a->state_bytes, cudaMemcpyDeviceToDevice, h->stream));
+  if (int rc = vf::handle_ready(h)) return afail(a, rc, std::string("forward step: ") + h->err);
   a->dts.assign(a->n_steps, 0.0);
   a->ts.assign(a->n_steps, 0.0);
+  bool stepwise = false;
+  if (frozen_dts) {
+    for (int n = 0; n < a->n_steps; ++n)
+      if (!(frozen_dts[n] >= 0)) return afail(a, VF_EINVAL, "forward step: dt must be >= 0");
+    std::memcpy(a->dts.data(), frozen_dts, sizeof(double) * a->n_steps);
+    if (int rc = forward_frozen(a)) return rc;
+  } else {
+    // A Float32 simulator's clock advances in Float32, this run's start times in
+    // Float64: step by step where a source reads the time.
+    stepwise = h->elem == 4 && h->af.p.any_dynamic;
+    if (!stepwise) {
+      if (int rc = forward_cfl(a)) return rc;
+      // an unbounded dt (a domain without waves) ends the device loop early
+      for (double dt : a->dts) stepwise = stepwise || !std::isfinite(dt);
+    }
+    if (stepwise)
+      if (int rc = forward_stepwise(a)) return rc;
+  }
   double t = 0.0;
   for (int n = 0; n < a->n_steps; ++n) {
     a->ts[n] = t;
-    if (n % a->K == 0)
-      VF_ACK(a, cudaMemcpyAsync(off(a->ckpt, (size_t)(n / a->K) * a->state_bytes), h->U[0], a->state_bytes,
-                                cudaMemcpyDeviceToDevice, h->stream));
-    int rc;
-    double dt = 0;
-    if (frozen_dts) {
-      dt = frozen_dts[n];
-      rc = vf_step_fixed(h, dt, t);
-    } else {
-      rc = vf_step(h, INFINITY, t, &dt);
-    }
-    if (rc) return afail(a, rc, std::string("forward step: ") + h->err);
-    a->dts[n] = dt;
-    t += dt;
+    t += a->dts[n];
   }
   if (dts_out) std::memcpy(dts_out, a->dts.data(), sizeof(double) * a->n_steps);
   a->have_forward = true;

@@ -49,6 +49,9 @@ int handle_ready(vf_handle* h);
 // loop's record (t0, end time, match_endtime, maximum_timestep < 0: none) to
 // the device on the handle's stream.
 int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep);
+// Copies the step record to the host (h->rec_h) and waits for the stream; an
+// error when a bounded wait of a step gave up.
+int handle_pull_record(vf_handle* h);
 // Enqueue n steps with global indices first, first+1, ... on the handle's
 // stream (a step whose record slot is inactive does nothing).
 int handle_enqueue_steps(vf_handle* h, long long first, int n);

@@ -60,19 +60,20 @@ cudaError_t ensemble_max_clusters_f32(int csize, int variant, int* out);
 cudaError_t launch_sample(const Geom<double>& g, const double* U, const int* ij, int n, double* out, cudaStream_t st);
 cudaError_t launch_sample(const Geom<float>& g, const float* U, const int* ij, int n, float* out, cudaStream_t st);
 // Adjoint kernels (vf_adjoint.cuh), one launch each; *nblocks_out receives the
-// number of dLoss/dCz partials k_adj_point wrote.
+// number of dLoss/dCz sums k_adj_point keeps.
 cudaError_t launch_adj_point(const AdjArgs<double>& a, int* nblocks_out, cudaStream_t st);
 cudaError_t launch_adj_point(const AdjArgs<float>& a, int* nblocks_out, cudaStream_t st);
-cudaError_t launch_adj_recon(const AdjArgs<double>& a, int dir, cudaStream_t st);
-cudaError_t launch_adj_recon(const AdjArgs<float>& a, int dir, cudaStream_t st);
+cudaError_t launch_adj_face(const AdjArgs<double>& a, cudaStream_t st);
+cudaError_t launch_adj_recon(const AdjArgs<double>& a, cudaStream_t st);
+cudaError_t launch_adj_face(const AdjArgs<float>& a, cudaStream_t st);
+cudaError_t launch_adj_recon(const AdjArgs<float>& a, cudaStream_t st);
 cudaError_t launch_adj_gather(const AdjArgs<double>& a, cudaStream_t st);
 cudaError_t launch_adj_gather(const AdjArgs<float>& a, cudaStream_t st);
-cudaError_t launch_adj_corner(const AdjArgs<double>& a, cudaStream_t st);
-cudaError_t launch_adj_corner(const AdjArgs<float>& a, cudaStream_t st);
 cudaError_t launch_adj_seed(const Geom<double>& g, const double* U, double* lam, const int* gi, const int* gj,
                             const double* target, int n, double* loss, cudaStream_t st);
 cudaError_t launch_adj_seed(const Geom<float>& g, const float* U, float* lam, const int* gi, const int* gj,
                             const double* target, int n, double* loss, cudaStream_t st);
+cudaError_t launch_adj_record(StepRecord* rec, double dt, double t, cudaStream_t st);
 cudaError_t launch_adj_sum(const double* part, int n, double* acc, cudaStream_t st);
 // Float64 quotients a[i] / b[i] as the Float64 kernels compute them (self-test).
 cudaError_t launch_selftest_quotients(const double* a, const double* b, int n, double* q, cudaStream_t st);

@@ -216,29 +216,23 @@ cudaError_t launch_adj_point_impl(const AdjArgs<T>& a, int* nblocks_out, cudaStr
 }
 
 template <typename T>
-cudaError_t launch_adj_recon_impl(const AdjArgs<T>& a, int dir, cudaStream_t st) {
+cudaError_t launch_adj_face_impl(const AdjArgs<T>& a, cudaStream_t st) {
   const dim3 blk(32, 4);
-  if (dir == 0) {
-    const dim3 grid((a.g.nx + 2 + 31) / 32, (a.g.ny + 3) / 4);
-    k_adj_recon<T, 0><<<grid, blk, 0, st>>>(a);
-  } else {
-    const dim3 grid((a.g.ny + 2 + 31) / 32, (a.g.nx + 3) / 4);
-    k_adj_recon<T, 1><<<grid, blk, 0, st>>>(a);
-  }
+  k_adj_face<T><<<dim3((a.g.nx + 1 + 31) / 32, (a.g.ny + 1 + 3) / 4, 2), blk, 0, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_adj_recon_impl(const AdjArgs<T>& a, cudaStream_t st) {
+  const dim3 blk(32, 4);
+  k_adj_recon<T><<<dim3((a.g.nx + 2 + 31) / 32, (a.g.ny + 2 + 3) / 4, 2), blk, 0, st>>>(a);
   return cudaGetLastError();
 }
 
 template <typename T>
 cudaError_t launch_adj_gather_impl(const AdjArgs<T>& a, cudaStream_t st) {
   const dim3 blk(32, 8);
-  k_adj_gather<T><<<dim3((a.g.nx + 31) / 32, (a.g.ny + 7) / 8), blk, 0, st>>>(a);
-  return cudaGetLastError();
-}
-
-template <typename T>
-cudaError_t launch_adj_corner_impl(const AdjArgs<T>& a, cudaStream_t st) {
-  const dim3 blk(32, 8);
-  k_adj_corner<T><<<dim3((a.g.N1 + 1 + 31) / 32, (a.g.N2 + 1 + 7) / 8), blk, 0, st>>>(a);
+  k_adj_gather<T><<<dim3((a.g.N1 + 1 + 31) / 32, (a.g.N2 + 1 + 7) / 8, 2), blk, 0, st>>>(a);
   return cudaGetLastError();
 }
 
