@@ -234,17 +234,17 @@ void make_tma_maps(vf_handle* h) {
   const long long nxp = vf::XOFF + h->N1;  // columns 0..XOFF-1 are padding
   bool ok = true;
   for (int k = 0; k < 2; ++k) {
-    ok = ok && encode_f64(&t.U[k], h->U[k], nxp, h->N2, h->P, h->PS, 3, vf::HX, vf::HY);
+    ok = ok && encode_f64(&t.U[k], h->U[k], nxp, h->N2, h->P, h->PS, 3, vf::TmaTile::HX, vf::TmaTile::HY);
     // tile stores: extent ends at the last interior row and at or before the last interior column
     ok = ok && encode_f64(&t.Ust[k], h->U[k], vf::tma_store_cols(vf::XOFF + h->cfg.gc + h->cfg.nx),
-                          h->cfg.gc + h->cfg.ny, h->P, h->PS, 3, vf::TX, vf::TY);
+                          h->cfg.gc + h->cfg.ny, h->P, h->PS, 3, vf::TmaTile::TX, vf::TmaTile::TY);
     t.Ub[k] = h->U[k];
   }
-  ok = ok && encode_f64(&t.L, h->L, nxp, h->N2, h->P, h->PS, 3, vf::HX, vf::HY);
+  ok = ok && encode_f64(&t.L, h->L, nxp, h->N2, h->P, h->PS, 3, vf::TmaTile::HX, vf::TmaTile::HY);
   t.Lb = h->L;
-  if (h->S) ok = ok && encode_f64(&t.S, h->S, nxp, h->N2, h->P, h->PS, 1, vf::HX, vf::HY);
+  if (h->S) ok = ok && encode_f64(&t.S, h->S, nxp, h->N2, h->P, h->PS, 1, vf::TmaTile::HX, vf::TmaTile::HY);
   t.Sb = h->S;
-  if (h->B) ok = ok && encode_f64(&t.B, h->B, nxp + 1, h->N2 + 1, h->PB, 0, 1, vf::BHX, vf::BHY);
+  if (h->B) ok = ok && encode_f64(&t.B, h->B, nxp + 1, h->N2 + 1, h->PB, 0, 1, vf::TmaTile::BHX, vf::TmaTile::BHY);
   t.Bb = h->B;
   t.ok = ok ? 1 : 0;
 }

@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(NT, EnsBlocks<T>::value) k_ensemble(const EnsI
         strip_setup_at(g, seg, u % nstrips, u / nstrips, s);
         flux_march_unit<T, true>(g, p, U0, sit.B, sit.L, sit.S, s, mx, my);
       }
-      block_key_max(mx, my, red, kx, ky);
+      block_key_max<NT>(mx, my, red, kx, ky);
     } else {
       T mx = (T)0, my = (T)0;
       for (int tile = (int)rank; tile < ntiles; tile += csize) {
@@ -188,7 +188,7 @@ __global__ void __launch_bounds__(NT, EnsBlocks<T>::value) k_ensemble(const EnsI
                            sm.f, t, mx, my);
         __syncthreads();
       }
-      block_speed_keys<T>(mx, my, red, kx, ky);
+      block_speed_keys<T, NT>(mx, my, red, kx, ky);
     }
     if (tid == 0) {
       slot.kx = kx;

@@ -74,7 +74,6 @@ cudaError_t launch_selftest_roots(const double* x, int n, double* sq, double* cb
 }
 
 cudaError_t configure_kernels_f64() {
-  const cudaError_t e = configure_impl<double>();
-  return e != cudaSuccess ? e : vf_faithful_configure();
+  return configure_impl<double>();
 }
 }  // namespace vf

@@ -37,18 +37,3 @@ cudaError_t vf_faithful_launch_flux(const void* a, const double* Uin, int parity
 cudaError_t vf_faithful_launch_stage(const void* a, const double* Uin, double* Uout, int parity, cudaStream_t st) {
   return vf_faithful::launch_stage_impl<double>(args_of(a), Uin, Uout, parity, st);
 }
-cudaError_t vf_faithful_configure() {
-  using namespace vf_faithful;
-  cudaError_t e = cudaFuncSetAttribute(k_flux<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)sizeof(SmemFlux<double>));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_stage2<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SmemStage<double>));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_flux_tma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SmemFlux<double>));
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(k_stage2_tma<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sizeof(SmemStage<double>));
-  return e;
-}

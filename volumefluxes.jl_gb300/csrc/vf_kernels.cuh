@@ -15,7 +15,7 @@
 //               (src/simulator.jl:147-150) and is computed on the device.
 //   apply pass  (forward Euler) the pointwise stage-1 update alone.
 //
-// Tiles are TX x TY interior cells; each block stages its tile with a 2-cell
+// Tiles are TX x TY interior cells (TileShape); each block stages its tile with a 2-cell
 // halo of (w, hu, hv) and a 2..3-cell halo of bottom corners in shared memory.
 // The Float64 kernels of the per-step path (k_flux_tma, k_stage2_tma) stage
 // them with TMA copies, and the stage pass writes its output tile with a TMA
@@ -27,20 +27,36 @@
 
 namespace vf {
 
-constexpr int TX = 32;
-constexpr int TY = 16;
-constexpr int NT = 256;
-constexpr int CPT = TX * TY / NT;  // cells per thread
-constexpr int HX = TX + 4;
-constexpr int HY = TY + 4;
-constexpr int BHX = TX + 6;  // TX + 5 corner columns are read; one more keeps Float64 rows 16-byte multiples
-constexpr int BHY = TY + 5;
-constexpr int LRN = (TX + 2) * TY > TX * (TY + 2) ? (TX + 2) * TY : TX * (TY + 2);
-constexpr int FN = (TX + 1) * TY > TX * (TY + 1) ? (TX + 1) * TY : TX * (TY + 1);
+// Tile of X x Y interior cells worked on by N threads, of which B blocks are to
+// fit on an SM (launch bounds). D: the x and the y direction at the same time,
+// half of the warps each, instead of one after the other.
+template <int X, int Y, int N, int B, bool D>
+struct TileShape {
+  static constexpr int TX = X, TY = Y, NT = N, MINB = B;
+  static constexpr bool SPLIT = D;
+  static constexpr int DIRS = D ? 2 : 1;               // buffers of face values and fluxes
+  static constexpr int CPT = (TX * TY + NT - 1) / NT;  // cells per thread
+  static constexpr int HX = TX + 4, HY = TY + 4;
+  static constexpr int BHX = TX + 6;  // TX + 5 corner columns are read; one more keeps Float64 rows 16-byte multiples
+  static constexpr int BHY = TY + 5;
+  static constexpr int LRN = (TX + 2) * TY > TX * (TY + 2) ? (TX + 2) * TY : TX * (TY + 2);
+  static constexpr int FN = (TX + 1) * TY > TX * (TY + 1) ? (TX + 1) * TY : TX * (TY + 1);
+};
+using BigTile = TileShape<32, 16, 256, 1, false>;  // Float32, and the ensemble in both precisions
+// Float64: 288 threads hold every phase of a 16x16 tile in one pass (18 x 16
+// cells reconstructed), in 72 registers and 40 KB, so 27 warps of three blocks
+// share an SM and wait at one another's barriers less than 24 warps of 32x16
+// tiles: 2.36 instead of 2.41 ms per step at 2048^2, 0.68 / 0.73 at 1024^2,
+// 0.241 / 0.292 at 512^2, 0.084 / 0.115 at 256^2 (two blocks of 112 registers:
+// 2.49 ms at 2048^2). 8x8 tiles with the directions side by side halve the
+// chain of phases that bounds a grid of few tiles: 37 instead of 62 us per step
+// up to 96^2, 47 / 59 at 160x128, 59 / 59 at 192^2, 105 / 84 at 256^2 (32x16
+// tiles: 117 us up to 256^2, 8 tiles for 64^2).
+using SmallTile = TileShape<16, 16, 288, 3, false>;
+using TinyTile = TileShape<8, 8, 192, 4, true>;
+constexpr int TX = BigTile::TX, TY = BigTile::TY, NT = BigTile::NT;
+constexpr int HX = BigTile::HX, HY = BigTile::HY, BHX = BigTile::BHX, BHY = BigTile::BHY;
 constexpr int XOFF = 2;  // leading pad columns in device rows
-#ifndef VF_TILE_MIN_BLOCKS
-#define VF_TILE_MIN_BLOCKS 1
-#endif
 
 // Device-resident step record. Slots indexed by step parity let every kernel
 // of step n read slot n&1 while the stage pass prepares slot (n+1)&1.
@@ -102,12 +118,12 @@ __device__ __forceinline__ T gld(const T* ptr) {
 // Bottom topography seen from a tile; (lx, ly) are tile-local cell coordinates,
 // corner (x0+lx, y0+ly) lives at sB[(ly+2)*BHX + lx+2]. Lookups follow
 // src/bottom_topography.jl:97-101.
-template <typename T>
+template <typename T, typename S = BigTile>
 struct BTile {
   const T* sB;
   int is_const;
   T c;
-  __device__ __forceinline__ T cn(int lx, int ly) const { return sB[(ly + 2) * BHX + lx + 2]; }
+  __device__ __forceinline__ T cn(int lx, int ly) const { return sB[(ly + 2) * S::BHX + lx + 2]; }
   __device__ __forceinline__ T cell(int lx, int ly) const {
     if (is_const) return c;
     return quarter<T>(((cn(lx, ly) + cn(lx + 1, ly)) + cn(lx, ly + 1)) + cn(lx + 1, ly + 1));
@@ -124,8 +140,9 @@ struct BTile {
   }
 };
 
-template <typename T>
+template <typename S, typename T>
 __device__ __forceinline__ void load_corners(const Geom<T>& g, const T* __restrict__ B, T* sB, int x0, int y0) {
+  constexpr int BHX = S::BHX, BHY = S::BHY, NT = S::NT;
   for (int idx = threadIdx.x; idx < BHX * BHY; idx += NT) {
     const int bx = idx % BHX, by = idx / BHX;
     const int cx = x0 - 2 + bx, cy = y0 - 2 + by;
@@ -163,133 +180,124 @@ __device__ __forceinline__ void u1_global(const Geom<T>& g, const Phys<T>& p, T 
                   gld<CG>(Lin + g.PS + o), gld<CG>(Lin + 2 * g.PS + o), S, Bc, w, hu, hv);
 }
 
-// Time derivative of one stage on the tile held in sU (3 planes of HY x HX).
+// Time derivative of one stage on the tile held in sU (3 planes of HY x HX),
+// direction by direction in three phases: reconstruct the tile's cells and one
+// layer on either side along DIR, the faces between them, the flux differences
+// and the bottom source. src/system.jl:64-70 (directions in order),
+// numericalflux.jl:21-33, linearreconstruction.jl:58-102,
+// source_term_bottom.jl:24-41. tid of nt threads take part.
+//
+// x: cells lx in [-1, TX], ly in [0, TY); y: cells lx in [0, TX), ly in [-1, TY].
+template <typename S, typename T, int DIR>
+__device__ __forceinline__ void tile_recon(const Phys<T>& p, const T* sU, const BTile<T, S>& bt, T* sL, T* sR, int tid,
+                                           int nt) {
+  constexpr int TX = S::TX, TY = S::TY, HX = S::HX, HY = S::HY, LRN = S::LRN;
+  constexpr int W = DIR == 0 ? TX + 2 : TX, N = W * (DIR == 0 ? TY : TY + 2), STEP = DIR == 0 ? 1 : HX;
+  for (int idx = tid; idx < N; idx += nt) {
+    const int lx = DIR == 0 ? idx % W - 1 : idx % W, ly = DIR == 0 ? idx / W : idx / W - 1;
+    const int c = (ly + 2) * HX + lx + 2;
+    T l[3], m[3], r[3], L[3], R[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      l[k] = sU[k * HX * HY + c - STEP];
+      m[k] = sU[k * HX * HY + c];
+      r[k] = sU[k * HX * HY + c + STEP];
+    }
+    if (p.rec_none) {
+      no_reconstruction<T>(m, bt.cell(lx, ly), L, R);
+    } else {
+      reconstruct_cell<T>(p, l, m, r, bt.template face_l<DIR>(lx, ly), bt.template face_r<DIR>(lx, ly), L, R);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      sL[k * LRN + idx] = L[k];
+      sR[k * LRN + idx] = R[k];
+    }
+  }
+}
+
+// Faces f between cells f-1 and f: x: f in [0, TX]; y: f in [0, TY].
+template <typename S, typename T, int DIR, bool SPEED>
+__device__ __forceinline__ void tile_faces(const Phys<T>& p, const T* sL, const T* sR, T* sF, T& mx, int nvx, int nvy,
+                                           int tid, int nt) {
+  constexpr int TX = S::TX, TY = S::TY, LRN = S::LRN, FN = S::FN;
+  constexpr int W = DIR == 0 ? TX + 1 : TX, N = W * (DIR == 0 ? TY : TY + 1);
+  for (int idx = tid; idx < N; idx += nt) {
+    const int fx = idx % W, fy = idx / W;
+    const int im = DIR == 0 ? fy * (TX + 2) + fx : idx, ip = im + (DIR == 0 ? 1 : TX);
+    T F0, F1, F2, sp = (T)0;
+    cu_face<T, DIR, SPEED>(p, sR[im], sR[LRN + im], sR[2 * LRN + im], sL[ip], sL[LRN + ip], sL[2 * LRN + ip], F0, F1,
+                           F2, sp);
+    sF[idx] = F0;
+    sF[FN + idx] = F1;
+    sF[2 * FN + idx] = F2;
+    if (SPEED && (DIR == 0 ? fy < nvy && fx <= nvx : fx < nvx && fy <= nvy)) mx = speed_max<T>(mx, sp);
+  }
+}
+
 // acc[k][*] receives -(1/Δx)(F_r-F_l) [+ bottom x], then -(1/Δy)(G_r-G_l)
 // [+ bottom y] for the cells this thread owns (cell tid + k*NT, x fastest).
-// src/system.jl:64-70 (directions in order), numericalflux.jl:21-33,
-// linearreconstruction.jl:58-102, source_term_bottom.jl:24-41.
-template <typename T, bool SPEED>
-__device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, const BTile<T>& bt, T* sL, T* sR, T* sF,
-                                                T (&acc)[CPT][3], T& mx, T& my, int nvx, int nvy) {
+template <typename S, typename T, int DIR>
+__device__ __forceinline__ void tile_accumulate(const Phys<T>& p, const BTile<T, S>& bt, const T* sL, const T* sR,
+                                                const T* sF, T (&acc)[S::CPT][3]) {
+  constexpr int TX = S::TX, TY = S::TY, NT = S::NT, CPT = S::CPT, FN = S::FN;
+  constexpr int STEP = DIR == 0 ? 1 : TX, M = DIR == 0 ? 1 : 2;
+#pragma unroll
+  for (int k = 0; k < CPT; ++k) {
+    const int c = threadIdx.x + k * NT;
+    if (CPT * NT > TX * TY && c >= TX * TY) break;
+    const int lx = c % TX, ly = c / TX;
+    const int fl = DIR == 0 ? ly * (TX + 1) + lx : c;
+    if constexpr (std::is_same<T, double>::value) {
+      T v[3];
+#pragma unroll
+      for (int j = 0; j < 3; ++j) v[j] = sF[j * FN + fl + STEP] - sF[j * FN + fl];
+      over_delta<DIR>(p, v);
+#pragma unroll
+      for (int j = 0; j < 3; ++j) acc[k][j] = DIR == 0 ? exact::zero_minus(v[j]) : acc[k][j] - v[j];
+    } else {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        acc[k][j] = (DIR == 0 ? (T)0 : acc[k][j]) -
+                    (DIR == 0 ? p.inv_dx : p.inv_dy) * (sF[j * FN + fl + STEP] - sF[j * FN + fl]);
+    }
+    const int rc = DIR == 0 ? ly * (TX + 2) + lx + 1 : c + TX;
+    for (int b = 0; b < p.n_bottom; ++b) {
+      const T Bl = bt.template face_l<DIR>(lx, ly), Br = bt.template face_r<DIR>(lx, ly);
+      acc[k][M] = acc[k][M] + p.neg_g * bottom_slope<T, DIR>(p, Br - Bl) * halve<T>(sR[rc] + sL[rc]);
+    }
+  }
+}
+
+template <typename S, typename T, bool SPEED>
+__device__ __forceinline__ void tile_derivative(const Phys<T>& p, const T* sU, const BTile<T, S>& bt, T* sL, T* sR,
+                                                T* sF, T (&acc)[S::CPT][3], T& mx, T& my, int nvx, int nvy) {
+  constexpr int NT = S::NT;
   const int tid = threadIdx.x;
-  // ---- x: reconstruct cells lx in [-1, TX], ly in [0, TY)
-  for (int idx = tid; idx < (TX + 2) * TY; idx += NT) {
-    const int lx = idx % (TX + 2) - 1, ly = idx / (TX + 2);
-    const int c = (ly + 2) * HX + lx + 2;
-    T l[3], m[3], r[3], L[3], R[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      l[k] = sU[k * HX * HY + c - 1];
-      m[k] = sU[k * HX * HY + c];
-      r[k] = sU[k * HX * HY + c + 1];
-    }
-    if (p.rec_none) {
-      no_reconstruction<T>(m, bt.cell(lx, ly), L, R);
-    } else {
-      reconstruct_cell<T>(p, l, m, r, bt.template face_l<0>(lx, ly), bt.template face_r<0>(lx, ly), L, R);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      sL[k * LRN + idx] = L[k];
-      sR[k * LRN + idx] = R[k];
-    }
-  }
-  __syncthreads();
-  // ---- x: faces f in [0, TX] between cells f-1 and f
-  for (int idx = tid; idx < (TX + 1) * TY; idx += NT) {
-    const int f = idx % (TX + 1), ly = idx / (TX + 1);
-    const int im = ly * (TX + 2) + f, ip = im + 1;
-    T F0, F1, F2, sp = (T)0;
-    cu_face<T, 0, SPEED>(p, sR[im], sR[LRN + im], sR[2 * LRN + im], sL[ip], sL[LRN + ip], sL[2 * LRN + ip], F0, F1, F2,
-                         sp);
-    sF[idx] = F0;
-    sF[FN + idx] = F1;
-    sF[2 * FN + idx] = F2;
-    if (SPEED && ly < nvy && f <= nvx) mx = speed_max<T>(mx, sp);
-  }
-  __syncthreads();
-  // ---- x: accumulate
-#pragma unroll
-  for (int k = 0; k < CPT; ++k) {
-    const int c = tid + k * NT;
-    const int lx = c % TX, ly = c / TX;
-    const int fl = ly * (TX + 1) + lx;
-    if constexpr (std::is_same<T, double>::value) {
-      T v[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) v[j] = sF[j * FN + fl + 1] - sF[j * FN + fl];
-      over_delta<0>(p, v);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) acc[k][j] = exact::zero_minus(v[j]);
-    } else {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) acc[k][j] = (T)0 - p.inv_dx * (sF[j * FN + fl + 1] - sF[j * FN + fl]);
-    }
-    const int rc = ly * (TX + 2) + lx + 1;
-    for (int b = 0; b < p.n_bottom; ++b) {
-      const T Bl = bt.template face_l<0>(lx, ly), Br = bt.template face_r<0>(lx, ly);
-      acc[k][1] = acc[k][1] + p.neg_g * bottom_slope<T, 0>(p, Br - Bl) * halve<T>(sR[rc] + sL[rc]);
-    }
-  }
-  __syncthreads();
-  // ---- y: reconstruct cells lx in [0, TX), ly in [-1, TY]
-  for (int idx = tid; idx < TX * (TY + 2); idx += NT) {
-    const int lx = idx % TX, ly = idx / TX - 1;
-    const int c = (ly + 2) * HX + lx + 2;
-    T l[3], m[3], r[3], L[3], R[3];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      l[k] = sU[k * HX * HY + c - HX];
-      m[k] = sU[k * HX * HY + c];
-      r[k] = sU[k * HX * HY + c + HX];
-    }
-    if (p.rec_none) {
-      no_reconstruction<T>(m, bt.cell(lx, ly), L, R);
-    } else {
-      reconstruct_cell<T>(p, l, m, r, bt.template face_l<1>(lx, ly), bt.template face_r<1>(lx, ly), L, R);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      sL[k * LRN + idx] = L[k];
-      sR[k * LRN + idx] = R[k];
-    }
-  }
-  __syncthreads();
-  // ---- y: faces f in [0, TY] between cells f-1 and f
-  for (int idx = tid; idx < TX * (TY + 1); idx += NT) {
-    const int lx = idx % TX, f = idx / TX;
-    const int im = f * TX + lx, ip = im + TX;
-    T F0, F1, F2, sp = (T)0;
-    cu_face<T, 1, SPEED>(p, sR[im], sR[LRN + im], sR[2 * LRN + im], sL[ip], sL[LRN + ip], sL[2 * LRN + ip], F0, F1, F2,
-                         sp);
-    sF[idx] = F0;
-    sF[FN + idx] = F1;
-    sF[2 * FN + idx] = F2;
-    if (SPEED && lx < nvx && f <= nvy) my = speed_max<T>(my, sp);
-  }
-  __syncthreads();
-  // ---- y: accumulate
-#pragma unroll
-  for (int k = 0; k < CPT; ++k) {
-    const int c = tid + k * NT;
-    const int lx = c % TX, ly = c / TX;
-    const int fl = ly * TX + lx;
-    if constexpr (std::is_same<T, double>::value) {
-      T v[3];
-#pragma unroll
-      for (int j = 0; j < 3; ++j) v[j] = sF[j * FN + fl + TX] - sF[j * FN + fl];
-      over_delta<1>(p, v);
-#pragma unroll
-      for (int j = 0; j < 3; ++j) acc[k][j] = acc[k][j] - v[j];
-    } else {
-#pragma unroll
-      for (int j = 0; j < 3; ++j) acc[k][j] = acc[k][j] - p.inv_dy * (sF[j * FN + fl + TX] - sF[j * FN + fl]);
-    }
-    const int rc = (ly + 1) * TX + lx;
-    for (int b = 0; b < p.n_bottom; ++b) {
-      const T Bl = bt.template face_l<1>(lx, ly), Br = bt.template face_r<1>(lx, ly);
-      acc[k][2] = acc[k][2] + p.neg_g * bottom_slope<T, 1>(p, Br - Bl) * halve<T>(sR[rc] + sL[rc]);
-    }
+  if constexpr (S::SPLIT) {
+    // x and y side by side, half of the warps each, with buffers of their own
+    constexpr int H = NT / 2;
+    T *yL = sL + 3 * S::LRN, *yR = sR + 3 * S::LRN, *yF = sF + 3 * S::FN;
+    if (tid < H) tile_recon<S, T, 0>(p, sU, bt, sL, sR, tid, H);
+    else tile_recon<S, T, 1>(p, sU, bt, yL, yR, tid - H, H);
+    __syncthreads();
+    if (tid < H) tile_faces<S, T, 0, SPEED>(p, sL, sR, sF, mx, nvx, nvy, tid, H);
+    else tile_faces<S, T, 1, SPEED>(p, yL, yR, yF, my, nvx, nvy, tid - H, H);
+    __syncthreads();
+    tile_accumulate<S, T, 0>(p, bt, sL, sR, sF, acc);
+    tile_accumulate<S, T, 1>(p, bt, yL, yR, yF, acc);
+  } else {
+    tile_recon<S, T, 0>(p, sU, bt, sL, sR, tid, NT);
+    __syncthreads();
+    tile_faces<S, T, 0, SPEED>(p, sL, sR, sF, mx, nvx, nvy, tid, NT);
+    __syncthreads();
+    tile_accumulate<S, T, 0>(p, bt, sL, sR, sF, acc);
+    __syncthreads();
+    tile_recon<S, T, 1>(p, sU, bt, sL, sR, tid, NT);
+    __syncthreads();
+    tile_faces<S, T, 1, SPEED>(p, sL, sR, sF, my, nvx, nvy, tid, NT);
+    __syncthreads();
+    tile_accumulate<S, T, 1>(p, bt, sL, sR, sF, acc);
   }
 }
 
@@ -317,14 +325,14 @@ __device__ __forceinline__ double speed_from_key<float>(unsigned long long k) {
 // ---------------------------------------------------------------------------
 // Flux pass: L(U0), S(U0) and the CFL maxima.
 // U and B come first: for Float64 both start 128-byte aligned (TMA destinations).
-template <typename T>
+template <typename T, typename S = BigTile>
 struct SmemFlux {
-  T U[3 * HX * HY];
-  T B[BHX * BHY];
-  T L[3 * LRN];
-  T R[3 * LRN];
-  T F[3 * FN];
-  unsigned long long red[2][NT / 32];
+  T U[3 * S::HX * S::HY];
+  T B[S::BHX * S::BHY];
+  T L[S::DIRS * 3 * S::LRN];
+  T R[S::DIRS * 3 * S::LRN];
+  T F[S::DIRS * 3 * S::FN];
+  unsigned long long red[2][S::NT / 32];
   T scal[8];
   unsigned long long bar;  // mbarrier of the tile copies
   int plain;               // 0: staged by TMA; 1: not staged (alignment); 2: the wait gave up
@@ -334,9 +342,10 @@ struct SmemFlux {
 // global memory; mx, my accumulate this thread's share of the CFL maxima.
 // t is the step's start time (time-dependent sources).
 // STAGED: s.U and s.B already hold the tile (TMA).
-template <typename T, bool CG, bool STAGED = false>
+template <typename T, bool CG, bool STAGED = false, typename S = BigTile>
 __device__ __forceinline__ void flux_tile(const Geom<T>& g, const Phys<T>& p, const T* U, const T* __restrict__ B,
-                                          T* Lout, T* Sout, int x0, int y0, SmemFlux<T>& s, double t, T& mx, T& my) {
+                                          T* Lout, T* Sout, int x0, int y0, SmemFlux<T, S>& s, double t, T& mx, T& my) {
+  constexpr int TX = S::TX, TY = S::TY, NT = S::NT, CPT = S::CPT, HX = S::HX, HY = S::HY;
   const int tid = threadIdx.x;
   const int nvx = min(TX, g.gc + g.nx - x0), nvy = min(TY, g.gc + g.ny - y0);
 
@@ -349,20 +358,20 @@ __device__ __forceinline__ void flux_tile(const Geom<T>& g, const Phys<T>& p, co
 #pragma unroll
       for (int k = 0; k < 3; ++k) s.U[k * HX * HY + idx] = ok ? gld<CG>(U + k * g.PS + o) : (T)0;
     }
-    if (!g.bottom_const) load_corners(g, B, s.B, x0, y0);
+    if (!g.bottom_const) load_corners<S>(g, B, s.B, x0, y0);
   }
   if (p.any_dynamic && tid == 0) point_scalars<T>(p, t, s.scal);
   __syncthreads();
 
-  BTile<T> bt{s.B, g.bottom_const, g.bconst};
+  BTile<T, S> bt{s.B, g.bottom_const, g.bconst};
   T acc[CPT][3];
-  tile_derivative<T, true>(p, s.U, bt, s.L, s.R, s.F, acc, mx, my, nvx, nvy);
+  tile_derivative<S, T, true>(p, s.U, bt, s.L, s.R, s.F, acc, mx, my, nvx, nvy);
 
 #pragma unroll
   for (int k = 0; k < CPT; ++k) {
     const int c = tid + k * NT;
     const int lx = c % TX, ly = c / TX;
-    if (lx >= nvx || ly >= nvy) continue;
+    if (lx >= nvx || ly >= nvy) continue;  // also the threads past the tile (ly >= TY >= nvy)
     const long long o = sidx(g, x0 + lx, y0 + ly);
     acc[k][0] = p.any_dynamic ? add_point_sources<T>(p, acc[k][0], s.scal, o) : add_point_sources<T>(p, acc[k][0]);
 #pragma unroll
@@ -379,6 +388,7 @@ __device__ __forceinline__ void flux_tile(const Geom<T>& g, const Phys<T>& p, co
 
 // Block maximum of per-thread CFL speed keys (IEEE bit patterns of speeds
 // >= 0): warp shuffles, then one shared-memory pass; valid in thread 0.
+template <int NT>
 __device__ __forceinline__ void block_key_max(unsigned long long kx, unsigned long long ky,
                                               unsigned long long (*red)[NT / 32], unsigned long long& kx_out,
                                               unsigned long long& ky_out) {
@@ -405,26 +415,26 @@ __device__ __forceinline__ void block_key_max(unsigned long long kx, unsigned lo
   }
 }
 
-template <typename T>
+template <typename T, int NT>
 __device__ __forceinline__ void block_speed_keys(T mx, T my, unsigned long long (*red)[NT / 32],
                                                  unsigned long long& kx_out, unsigned long long& ky_out) {
-  block_key_max(speed_key<T>(mx), speed_key<T>(my), red, kx_out, ky_out);
+  block_key_max<NT>(speed_key<T>(mx), speed_key<T>(my), red, kx_out, ky_out);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS) k_flux(Geom<T> g, Phys<T> p, const T* __restrict__ U, const T* __restrict__ B,
+template <typename T, typename S>
+__global__ void __launch_bounds__(S::NT, S::MINB) k_flux(Geom<T> g, Phys<T> p, const T* __restrict__ U, const T* __restrict__ B,
                                              T* __restrict__ Lout, T* __restrict__ Sout, StepRecord* rec, int parity) {
   if (!rec->active[parity]) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemFlux<T>& s = *reinterpret_cast<SmemFlux<T>*>(smem_raw);
-  const int x0 = g.gc + blockIdx.x * TX, y0 = g.gc + blockIdx.y * TY;
+  SmemFlux<T, S>& s = *reinterpret_cast<SmemFlux<T, S>*>(smem_raw);
+  const int x0 = g.gc + blockIdx.x * S::TX, y0 = g.gc + blockIdx.y * S::TY;
   const double t = p.any_dynamic ? rec->t[parity] : 0.0;
   T mx = (T)0, my = (T)0;
-  flux_tile<T, false>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
+  flux_tile<T, false, false, S>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
 
   // CFL maxima: warp shuffle, then one atomic per block and direction.
   unsigned long long kx = 0, ky = 0;
-  block_speed_keys<T>(mx, my, s.red, kx, ky);
+  block_speed_keys<T, S::NT>(mx, my, s.red, kx, ky);
   if (threadIdx.x == 0) {
     atomicMax(&rec->speed_bits[parity][0], kx);
     atomicMax(&rec->speed_bits[parity][1], ky);
@@ -432,31 +442,31 @@ __global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS) k_flux(Geom<T> g, Phys
 }
 
 // Bytes of one staged tile of n planes, and of the corner tile.
-template <typename T>
-__host__ __device__ constexpr unsigned tile_bytes(int planes) { return (unsigned)(planes * HX * HY * sizeof(T)); }
-template <typename T>
-__host__ __device__ constexpr unsigned corner_bytes() { return (unsigned)(BHX * BHY * sizeof(T)); }
+template <typename T, typename S>
+__host__ __device__ constexpr unsigned tile_bytes(int planes) { return (unsigned)(planes * S::HX * S::HY * sizeof(T)); }
+template <typename T, typename S>
+__host__ __device__ constexpr unsigned corner_bytes() { return (unsigned)(S::BHX * S::BHY * sizeof(T)); }
 
 // k_flux with the tile staged by TMA (Float64). Thread 0 issues one 3D copy of
 // the three state planes and one 2D copy of the corners; everyone waits on the
 // mbarrier, then the flux pass runs as in k_flux.
-template <typename T>
-__global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS)
+template <typename T, typename S>
+__global__ void __launch_bounds__(S::NT, S::MINB)
     k_flux_tma(Geom<T> g, Phys<T> p, const __grid_constant__ CUtensorMap mU, const __grid_constant__ CUtensorMap mB,
                const T* __restrict__ U, const T* __restrict__ B, T* __restrict__ Lout, T* __restrict__ Sout,
                StepRecord* rec, int parity) {
   static_assert(sizeof(T) == 8, "TMA tiles are Float64 (the tile origin is 16-byte aligned only for 8-byte cells)");
   if (!rec->active[parity]) return;
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemFlux<T>& s = *reinterpret_cast<SmemFlux<T>*>(smem_raw);
-  const int x0 = g.gc + blockIdx.x * TX, y0 = g.gc + blockIdx.y * TY;
+  SmemFlux<T, S>& s = *reinterpret_cast<SmemFlux<T, S>*>(smem_raw);
+  const int x0 = g.gc + blockIdx.x * S::TX, y0 = g.gc + blockIdx.y * S::TY;
   const int cx = x0 - 2 + XOFF, cy = y0 - 2;
   if (threadIdx.x == 0) {
     const bool ok = tma_ok(cx, (int)sizeof(T), s.U) && (g.bottom_const || tma_ok(cx, (int)sizeof(T), s.B));
     s.plain = ok ? 0 : 1;
     if (ok) {
       mbar_init(&s.bar, 1);
-      mbar_expect_tx(&s.bar, tile_bytes<T>(3) + (g.bottom_const ? 0u : corner_bytes<T>()));
+      mbar_expect_tx(&s.bar, tile_bytes<T, S>(3) + (g.bottom_const ? 0u : corner_bytes<T, S>()));
       tma_load_3d(s.U, &mU, cx, cy, 0, &s.bar);
       if (!g.bottom_const) tma_load_2d(s.B, &mB, cx, cy, &s.bar);
     }
@@ -470,12 +480,12 @@ __global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS)
   const double t = p.any_dynamic ? rec->t[parity] : 0.0;
   T mx = (T)0, my = (T)0;
   if (s.plain)
-    flux_tile<T, false, false>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
+    flux_tile<T, false, false, S>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
   else
-    flux_tile<T, false, true>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
+    flux_tile<T, false, true, S>(g, p, U, B, Lout, Sout, x0, y0, s, t, mx, my);
 
   unsigned long long kx = 0, ky = 0;
-  block_speed_keys<T>(mx, my, s.red, kx, ky);
+  block_speed_keys<T, S::NT>(mx, my, s.red, kx, ky);
   if (threadIdx.x == 0) {
     atomicMax(&rec->speed_bits[parity][0], kx);
     atomicMax(&rec->speed_bits[parity][1], ky);
@@ -663,43 +673,45 @@ __device__ __forceinline__ void neumann_outer(const Geom<T>& g, const Phys<T>& p
 // ---------------------------------------------------------------------------
 // RK2 stage pass.
 // L, R and F come first and are contiguous: before the stage-2 derivative
-// overwrites them they hold the TMA-staged halo tiles of U0 (3 planes), L (3)
-// and S (1), STAGE_PLANES planes of HX x HY from offset 0 (k_stage2_tma).
-// For Float64 every TMA destination starts 128-byte aligned.
-template <typename T>
+// overwrites them they hold the TMA-staged halo tiles of U0 (3 planes) and L
+// (3), planes of HX x HY from offset 0; S is staged in the first plane of U1
+// (k_stage2_tma). For Float64 every TMA destination starts 128-byte aligned.
+template <typename T, typename S = BigTile>
 struct SmemStage {
-  T L[3 * LRN];
-  T R[3 * LRN];
-  T F[3 * FN];
-  T U1[3 * HX * HY];
-  T U0[3 * TX * TY];
-  T B[BHX * BHY];
+  T L[S::DIRS * 3 * S::LRN];
+  T R[S::DIRS * 3 * S::LRN];
+  T F[S::DIRS * 3 * S::FN];
+  T U1[3 * S::HX * S::HY];
+  T U0[3 * S::TX * S::TY];
+  T B[S::BHX * S::BHY];
   double dt;
   T scal[8];
   unsigned long long bar;  // mbarrier of the tile copies
   int plain;               // 0: staged by TMA; 1: not staged (alignment); 2: the wait gave up
 };
-constexpr int STAGE_PLANES = 7;
-static_assert(3 * LRN + 3 * LRN + 3 * FN >= STAGE_PLANES * HX * HY, "stage staging area must fit in L, R, F");
+using TmaTile = SmallTile;
+static_assert(6 * TmaTile::LRN + 3 * TmaTile::FN >= 6 * TmaTile::HX * TmaTile::HY,
+              "the staged planes of U0 and L must fit in L, R, F");
 
 // RK2 stage pass over one tile at (x0, y0) (block-collective): U2 with its
 // ghosts into Uo. dt is the step's dt, t its start time.
-// STAGED: the halo tiles of U0, L, S sit at the start of s (planes of HX x HY:
-// U0 0..2, L 3..5, S 6) and s.B holds the corners (TMA); the interior of U2
+// STAGED: the halo tiles of U0 and L sit at the start of s (planes of HX x HY:
+// U0 0..2, L 3..5), that of S in s.U1, and s.B holds the corners (TMA); the interior of U2
 // goes to s.U0 (in place: each thread overwrites the cells it read) for a
 // tensor store by the caller, its ghost copies straight to Uo.
-template <typename T, bool CG, bool STAGED = false>
+template <typename T, bool CG, bool STAGED = false, typename S = BigTile>
 __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, const T* U0, const T* __restrict__ B,
-                                            const T* Lin, const T* Sin, T* Uo, int x0, int y0, SmemStage<T>& s,
+                                            const T* Lin, const T* Sin, T* Uo, int x0, int y0, SmemStage<T, S>& s,
                                             double dt, double t) {
+  constexpr int TX = S::TX, TY = S::TY, NT = S::NT, CPT = S::CPT, HX = S::HX, HY = S::HY;
   const int tid = threadIdx.x;
   const int nvx = min(TX, g.gc + g.nx - x0), nvy = min(TY, g.gc + g.ny - y0);
   if (p.any_dynamic && tid == 1) point_scalars<T>(p, t, s.scal);
-  if (!STAGED && !g.bottom_const) load_corners(g, B, s.B, x0, y0);
+  if (!STAGED && !g.bottom_const) load_corners<S>(g, B, s.B, x0, y0);
   __syncthreads();
   const T* stg = s.L;  // staged planes (STAGED only)
   const T tdt = (T)dt;
-  BTile<T> bt{s.B, g.bottom_const, g.bconst};
+  BTile<T, S> bt{s.B, g.bottom_const, g.bconst};
 
   // U1 on tile + halo, from U0, L, S. Ghost cells take U1 of their boundary
   // source cell (src/bc.jl:29-40, 81-110), computed the same pointwise way;
@@ -711,7 +723,7 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
     const bool yin = gy >= g.gc && gy < g.gc + g.ny;
     T w = (T)0, hu = (T)0, hv = (T)0;
     if (xin && yin) {
-      T a0, a1, a2, l0, l1, l2, S;
+      T a0, a1, a2, l0, l1, l2, fr;
       if constexpr (STAGED) {
         constexpr int A = HX * HY;
         a0 = stg[idx];
@@ -720,7 +732,7 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
         l0 = stg[3 * A + idx];
         l1 = stg[4 * A + idx];
         l2 = stg[5 * A + idx];
-        S = p.friction ? stg[6 * A + idx] : (T)0;
+        fr = p.friction ? s.U1[idx] : (T)0;  // this thread writes U1[idx] below
       } else {
         const long long o = sidx(g, gx, gy);
         a0 = gld<CG>(U0 + o);
@@ -729,9 +741,9 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
         l0 = gld<CG>(Lin + o);
         l1 = gld<CG>(Lin + g.PS + o);
         l2 = gld<CG>(Lin + 2 * g.PS + o);
-        S = p.friction ? gld<CG>(Sin + o) : (T)0;
+        fr = p.friction ? gld<CG>(Sin + o) : (T)0;
       }
-      stage1_point<T>(p, tdt, a0, a1, a2, l0, l1, l2, S, bt.cell(lx, ly), w, hu, hv);
+      stage1_point<T>(p, tdt, a0, a1, a2, l0, l1, l2, fr, bt.cell(lx, ly), w, hu, hv);
       if (lx >= 0 && lx < TX && ly >= 0 && ly < TY) {
         const int t = ly * TX + lx;
         s.U0[t] = a0;
@@ -763,7 +775,7 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
 
   T acc[CPT][3];
   T mx = (T)0, my = (T)0;
-  tile_derivative<T, false>(p, s.U1, bt, s.L, s.R, s.F, acc, mx, my, nvx, nvy);
+  tile_derivative<S, T, false>(p, s.U1, bt, s.L, s.R, s.F, acc, mx, my, nvx, nvy);
 
 #pragma unroll
   for (int k = 0; k < CPT; ++k) {
@@ -798,8 +810,8 @@ __device__ __forceinline__ void stage2_tile(const Geom<T>& g, const Phys<T>& p, 
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS) k_stage2(Geom<T> g, Phys<T> p, const T* __restrict__ U0, const T* __restrict__ B,
+template <typename T, typename S>
+__global__ void __launch_bounds__(S::NT, S::MINB) k_stage2(Geom<T> g, Phys<T> p, const T* __restrict__ U0, const T* __restrict__ B,
                                                const T* __restrict__ Lin, const T* __restrict__ Sin, T* __restrict__ Uo,
                                                StepRecord* rec, int parity) {
   const bool root = blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0;
@@ -808,19 +820,19 @@ __global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS) k_stage2(Geom<T> g, Ph
     return;
   }
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  SmemStage<T>& s = *reinterpret_cast<SmemStage<T>*>(smem_raw);
-  const int x0 = g.gc + blockIdx.x * TX, y0 = g.gc + blockIdx.y * TY;
+  SmemStage<T, S>& s = *reinterpret_cast<SmemStage<T, S>*>(smem_raw);
+  const int x0 = g.gc + blockIdx.x * S::TX, y0 = g.gc + blockIdx.y * S::TY;
   if (threadIdx.x == 0) s.dt = step_dt<T>(g, rec, parity);
   __syncthreads();
   const double dt = s.dt;
-  stage2_tile<T, false>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
+  stage2_tile<T, false, false, S>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
   if (root) advance_record<T>(rec, parity, dt);
 }
 
 // k_stage2 with the halo tiles of U0, L, S and the corners staged by TMA
 // (Float64): three or four copies on one mbarrier, issued by thread 0.
-template <typename T>
-__global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS)
+template <typename T, typename S>
+__global__ void __launch_bounds__(S::NT, S::MINB)
     k_stage2_tma(Geom<T> g, Phys<T> p, const __grid_constant__ CUtensorMap mU, const __grid_constant__ CUtensorMap mL,
                  const __grid_constant__ CUtensorMap mS, const __grid_constant__ CUtensorMap mB,
                  const __grid_constant__ CUtensorMap mUo,
@@ -833,23 +845,23 @@ __global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS)
     return;
   }
   extern __shared__ __align__(128) unsigned char smem_raw[];
-  SmemStage<T>& s = *reinterpret_cast<SmemStage<T>*>(smem_raw);
-  const int x0 = g.gc + blockIdx.x * TX, y0 = g.gc + blockIdx.y * TY;
+  SmemStage<T, S>& s = *reinterpret_cast<SmemStage<T, S>*>(smem_raw);
+  const int x0 = g.gc + blockIdx.x * S::TX, y0 = g.gc + blockIdx.y * S::TY;
   const int cx = x0 - 2 + XOFF, cy = y0 - 2;
   if (threadIdx.x == 0) {
-    constexpr int A = HX * HY;
+    constexpr int A = S::HX * S::HY;
     T* stg = s.L;
     const bool ok = tma_ok(cx, (int)sizeof(T), stg) && tma_ok(cx, (int)sizeof(T), stg + 3 * A) &&
-                    tma_ok(cx, (int)sizeof(T), stg + 6 * A) && (g.bottom_const || tma_ok(cx, (int)sizeof(T), s.B)) &&
+                    tma_ok(cx, (int)sizeof(T), s.U1) && (g.bottom_const || tma_ok(cx, (int)sizeof(T), s.B)) &&
                     tma_ok(x0 + XOFF, (int)sizeof(T), s.U0);
     s.plain = ok ? 0 : 1;
     if (ok) {
       mbar_init(&s.bar, 1);
-      mbar_expect_tx(&s.bar, tile_bytes<T>(6) + (p.friction ? tile_bytes<T>(1) : 0u) +
-                                 (g.bottom_const ? 0u : corner_bytes<T>()));
+      mbar_expect_tx(&s.bar, tile_bytes<T, S>(6) + (p.friction ? tile_bytes<T, S>(1) : 0u) +
+                                 (g.bottom_const ? 0u : corner_bytes<T, S>()));
       tma_load_3d(stg, &mU, cx, cy, 0, &s.bar);
       tma_load_3d(stg + 3 * A, &mL, cx, cy, 0, &s.bar);
-      if (p.friction) tma_load_2d(stg + 6 * A, &mS, cx, cy, &s.bar);
+      if (p.friction) tma_load_2d(s.U1, &mS, cx, cy, &s.bar);
       if (!g.bottom_const) tma_load_2d(s.B, &mB, cx, cy, &s.bar);
     }
     s.dt = step_dt<T>(g, rec, parity);
@@ -862,9 +874,9 @@ __global__ void __launch_bounds__(NT, VF_TILE_MIN_BLOCKS)
   __syncthreads();
   const double dt = s.dt;
   if (s.plain) {
-    stage2_tile<T, false, false>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
+    stage2_tile<T, false, false, S>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
   } else {
-    stage2_tile<T, false, true>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
+    stage2_tile<T, false, true, S>(g, p, U0, B, Lin, Sin, Uo, x0, y0, s, dt, rec->t[parity]);
     // The interior tile from s.U0 (128-byte aligned, x0 + XOFF even) in one tensor store.
     fence_async_smem();
     __syncthreads();

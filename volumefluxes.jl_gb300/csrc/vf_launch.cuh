@@ -13,7 +13,6 @@
 cudaError_t vf_faithful_launch_step(const void* args, const double* Uin, double* Uout, int parity, cudaStream_t st);
 cudaError_t vf_faithful_launch_flux(const void* args, const double* Uin, int parity, cudaStream_t st);
 cudaError_t vf_faithful_launch_stage(const void* args, const double* Uin, double* Uout, int parity, cudaStream_t st);
-cudaError_t vf_faithful_configure();
 
 namespace vf {
 

@@ -34,15 +34,15 @@ constexpr int kMarchWarpsPerSM = 16;
 
 template <typename T>
 cudaError_t configure_impl() {
-  cudaError_t e = cudaFuncSetAttribute(k_flux<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemFlux<T>));
-  if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_stage2<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemStage<T>));
-  if (e != cudaSuccess) return e;
-  if constexpr (sizeof(T) == 8) {
-    e = cudaFuncSetAttribute(k_flux_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemFlux<T>));
+  cudaError_t e = cudaSuccess;
+  if constexpr (sizeof(T) == 4) {  // the Float64 tiles stay within the 48 KB that need no opt-in
+    e = cudaFuncSetAttribute(k_flux<T, BigTile>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemFlux<T>));
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_stage2_tma<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemStage<T>));
+    e = cudaFuncSetAttribute(k_stage2<T, BigTile>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SmemStage<T>));
     if (e != cudaSuccess) return e;
+  } else {
+    static_assert(sizeof(SmemStage<T, SmallTile>) <= 48 * 1024 && sizeof(SmemStage<T, TinyTile>) <= 48 * 1024, "");
   }
   e = cudaFuncSetAttribute(k_ensemble<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemEns<T>));
   if (e != cudaSuccess) return e;
@@ -137,49 +137,72 @@ int tma_volume(const StepArgs<T>& a, const T* Uin) {
   }
 }
 
+template <typename S, typename T>
+dim3 tile_grid(const Geom<T>& g) {
+  return dim3((g.nx + S::TX - 1) / S::TX, (g.ny + S::TY - 1) / S::TY);
+}
+// Float64 grids small enough that TinyTile leaves at most kTinyTilesPerSM
+// blocks to an SM: measured even with SmallTile at 3.8 (192^2), ahead at 2.1
+// (160x128: 47 against 59 us per step), behind at 6.7 (256^2).
+constexpr int kTinyTilesPerSM = 3;
+template <typename T>
+bool tiny_tiles(const Geom<T>& g) {
+  const dim3 t = tile_grid<TinyTile>(g);
+  return (long long)t.x * t.y <= 152LL * kTinyTilesPerSM;
+}
+template <typename S, typename T>
+cudaError_t launch_flux_tiles(const StepArgs<T>& a, const T* Uin, int parity, cudaStream_t st) {
+  k_flux<T, S><<<tile_grid<S>(a.g), S::NT, sizeof(SmemFlux<T, S>), st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity);
+  return cudaGetLastError();
+}
+template <typename S, typename T>
+cudaError_t launch_stage_tiles(const StepArgs<T>& a, const T* Uin, T* Uout, int parity, cudaStream_t st) {
+  k_stage2<T, S><<<tile_grid<S>(a.g), S::NT, sizeof(SmemStage<T, S>), st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec,
+                                                                            parity);
+  return cudaGetLastError();
+}
+
 template <typename T>
 cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cudaStream_t st) {
-  if constexpr (sizeof(T) == 8) {
-    const int v = tma_volume<T>(a, Uin);
-    if (v >= 0) {
-      const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
-      k_flux_tma<T><<<grid, NT, sizeof(SmemFlux<T>), st>>>(a.g, a.p, a.tma.U[v], a.tma.B, Uin, a.B, a.L, a.S, a.rec,
-                                                            parity);
-      return cudaGetLastError();
-    }
-  }
   if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::flux);
     k_flux_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
     return cudaGetLastError();
   }
-  const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
-  k_flux<T><<<grid, NT, sizeof(SmemFlux<T>), st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity);
-  return cudaGetLastError();
+  if constexpr (sizeof(T) == 8) {
+    if (tiny_tiles(a.g)) return launch_flux_tiles<TinyTile>(a, Uin, parity, st);
+    const int v = tma_volume<T>(a, Uin);
+    if (v < 0) return launch_flux_tiles<SmallTile>(a, Uin, parity, st);
+    k_flux_tma<T, TmaTile><<<tile_grid<TmaTile>(a.g), TmaTile::NT, sizeof(SmemFlux<T, TmaTile>), st>>>(
+        a.g, a.p, a.tma.U[v], a.tma.B, Uin, a.B, a.L, a.S, a.rec, parity);
+    return cudaGetLastError();
+  } else {
+    return launch_flux_tiles<BigTile>(a, Uin, parity, st);
+  }
 }
 
 template <typename T>
 cudaError_t launch_stage_impl(const StepArgs<T>& a, const T* Uin, T* Uout, int parity, cudaStream_t st) {
-  const dim3 grid((a.g.nx + TX - 1) / TX, (a.g.ny + TY - 1) / TY);
-  if (a.rk2 && a.variant == 0) {
+  if (!a.rk2) {
+    k_apply_fe<T><<<tile_grid<BigTile>(a.g), NT, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    return cudaGetLastError();
+  }
+  if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::stage);
     k_stage_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity,
                                                                     seg);
-  } else if (a.rk2) {
-    if constexpr (sizeof(T) == 8) {
-      const int v = tma_volume<T>(a, Uin);
-      if (v >= 0 && Uout == a.tma.Ub[v ^ 1]) {
-        k_stage2_tma<T><<<grid, NT, sizeof(SmemStage<T>), st>>>(a.g, a.p, a.tma.U[v], a.tma.L, a.tma.S, a.tma.B,
-                                                                 a.tma.Ust[v ^ 1], Uin, a.B, a.L, a.S, Uout, a.rec,
-                                                                 parity);
-        return cudaGetLastError();
-      }
-    }
-    k_stage2<T><<<grid, NT, sizeof(SmemStage<T>), st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
-  } else {
-    k_apply_fe<T><<<grid, NT, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    return cudaGetLastError();
   }
-  return cudaGetLastError();
+  if constexpr (sizeof(T) == 8) {
+    if (tiny_tiles(a.g)) return launch_stage_tiles<TinyTile>(a, Uin, Uout, parity, st);
+    const int v = tma_volume<T>(a, Uin);
+    if (v < 0 || Uout != a.tma.Ub[v ^ 1]) return launch_stage_tiles<SmallTile>(a, Uin, Uout, parity, st);
+    k_stage2_tma<T, TmaTile><<<tile_grid<TmaTile>(a.g), TmaTile::NT, sizeof(SmemStage<T, TmaTile>), st>>>(
+        a.g, a.p, a.tma.U[v], a.tma.L, a.tma.S, a.tma.B, a.tma.Ust[v ^ 1], Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    return cudaGetLastError();
+  } else {
+    return launch_stage_tiles<BigTile>(a, Uin, Uout, parity, st);
+  }
 }
 
 template <typename T>

@@ -34,11 +34,11 @@ namespace vf {
 // Tensor maps of one handle's buffers (Float64 tile kernels only). A launch
 // uses them only when its buffers are the ones the maps were made for.
 struct TmaMaps {
-  CUtensorMap U[2];  // the two state volumes: 3D (x, y, plane), box HX x HY x 3
-  CUtensorMap Ust[2];  // the same volumes for tile stores: interior extent only, box TX x TY x 3
+  CUtensorMap U[2];  // the two state volumes: 3D (x, y, plane), box TmaTile HX x HY x 3
+  CUtensorMap Ust[2];  // the same volumes for tile stores: interior extent only, box TmaTile TX x TY x 3
   CUtensorMap L;     // stage-1 derivative planes, same shape
-  CUtensorMap S;     // friction factor, 2D, box HX x HY
-  CUtensorMap B;     // bottom corners, 2D, box BHX x BHY
+  CUtensorMap S;     // friction factor, 2D, box TmaTile HX x HY
+  CUtensorMap B;     // bottom corners, 2D, box TmaTile BHX x BHY
   const void* Ub[2];
   const void* Lb;
   const void* Sb;
