@@ -242,14 +242,14 @@ int vf_selftest_near_dry_quotients(int32_t device, const float* a, const float* 
 #define VF_BATCH_MAX_STEPS 3   /* stopped after max_steps steps */
 
 typedef struct vf_batch_options {
-  int32_t tiles_per_cta;   /* target 32x16 tiles per CTA when sizing a cluster; 0: default (16) */
+  int32_t tiles_per_cta;   /* target 32x16 tiles per CTA when sizing a cluster; 0: default (4) */
   int32_t max_cluster;     /* largest cluster (1..16); 0: default (16) */
   double time_limit_s;     /* watchdog from the batch's start, in seconds; <= 0: default (600 s) */
   int32_t seg_rows;        /* rows per strip segment of Float32 column-marching members
-                              (8..256); 0: 64, halved down to 8 until every warp has two */
+                              (8..256); 0: 8 */
   int64_t wide_cells;      /* members with at least this many interior cells run the plain
                               whole-grid kernels on their own stream instead of a cluster;
-                              0: default (262144), < 0: never */
+                              0: default (8192 in Float64, 65536 in Float32), < 0: never */
 } vf_batch_options;
 
 typedef struct vf_batch vf_batch;

@@ -411,7 +411,8 @@ void destroy(vf_handle* h) {
 namespace vf {
 int handle_ready(vf_handle* h) { return ensure_ready(h); }
 
-int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep) {
+int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep,
+                      long long max_steps) {
   reset_record(h);
   vf::StepRecord* r = h->rec_h;
   r->t[0] = t0;
@@ -420,6 +421,7 @@ int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime
   r->has_max_ts = maximum_timestep >= 0 ? 1 : 0;
   r->max_ts = maximum_timestep;
   r->endtime = endtime;
+  r->max_steps = max_steps > 0 ? max_steps : 0;
   return push_record(h);
 }
 

@@ -11,9 +11,9 @@
 // host memory, so the host sees every simulation finish without synchronising
 // the launch it belongs to.
 //
-// Simulations of at least wide_cells interior cells (default 512^2) are
-// "wide": a 16-CTA cluster would leave most of the GPU to them alone and make
-// them the batch's tail, so they run the plain
+// Simulations of at least wide_cells interior cells (default 8192 in Float64,
+// 65536 in Float32; wide_cells_for) are "wide": a 16-CTA cluster would leave most
+// of the GPU to them alone and make them the batch's tail, so they run the plain
 // whole-grid step kernels on their handle's stream instead, as the device loop
 // of vf_simulate, in chunks of kChunk steps captured once as a CUDA graph.
 // kInFlight chunks are kept queued; after each, the step record is copied to pinned
@@ -44,7 +44,8 @@ namespace {
 struct Wide {
   int member = 0;
   long long enqueued = 0;      // steps enqueued so far
-  long long max_steps = 0;
+  long long max_steps = 0;     // the record's limit: the device stops there by itself
+  double endtime = 0;
   int head = 0, inflight = 0;  // chunks head .. head+inflight-1 are in flight; chunk c uses ev/rec slot c % 3
   long long chunk_end[3] = {0, 0, 0};
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
@@ -143,7 +144,7 @@ struct Opts {
 };
 
 Opts resolve(const vf_batch_options* o) {
-  Opts r{16, 16, 600.0, 0, 1LL << 18};
+  Opts r{4, 16, 600.0, 0, 0};
   if (o) {
     if (o->wide_cells > 0) r.wide_cells = o->wide_cells;
     if (o->wide_cells < 0) r.wide_cells = LLONG_MAX;
@@ -153,6 +154,23 @@ Opts resolve(const vf_batch_options* o) {
     if (o->seg_rows > 0) r.seg_rows = std::min(256, std::max(8, o->seg_rows));
   }
   return r;
+}
+
+// Interior cells from which a member runs the whole-grid kernels. It depends on
+// the member and the options alone, never on the batch: a Float32 member's bits
+// differ between the designs, and its result must not depend on the mix. The
+// plain kernels cut a grid into as many blocks as the GPU has room for, where a
+// cluster has 16 CTAs at most; clusters win only while members are small and
+// many. Makespan in ms, all members whole-grid / this threshold / clusters:
+//   Float64, 20 members of 64-224^2, 8 steps: 2.15 / - / 4.0; 8 of 64-160^2:
+//   0.85 / - / 1.75; 200 of 64-256^2, 20 steps: 52 / - / 65; but 200 of
+//   64-80^2, 40 steps: 52 / 42 / 42.
+//   Float32, 16 members of 64-448^2, 60 steps: 4.0 / 4.7 / 10.5; 40: 8.6 / 9.5 /
+//   11.3; 100, 24 steps: 9.9 / 6.6 / 6.7; 128 of 64-1024^2, 40 steps: 30.5 /
+//   28.6 / 29.2 (131072 cells: 7.0, 8.2, -, 28.9).
+long long wide_cells_for(const vf_handle* h, const Opts& o) {
+  if (o.wide_cells > 0) return o.wide_cells;
+  return h->elem == 8 ? 8192 : 65536;
 }
 
 // Kernel design of a member, as the plain path chooses it (vf_abi.cu
@@ -190,15 +208,9 @@ int fit_cluster(int device, int real_bytes, int variant, int c) {
   return 1;
 }
 
-// Rows per strip segment of a marching member: 64, halved (down to 8) until
-// the cluster's warps have at least two segments each.
-int seg_rows_for(const vf_handle* h, int csize, int fixed) {
-  if (fixed > 0) return fixed;
-  const int nstrips = (h->cfg.nx + vf::MOUT - 1) / vf::MOUT;
-  int seg = 64;
-  while (seg > 8 && (long long)nstrips * ((h->cfg.ny + seg - 1) / seg) < 2LL * csize * (vf::NT / 32)) seg /= 2;
-  return seg;
-}
+// Rows per strip segment of a marching member: 8 (16 rows measured 4.6 instead
+// of 4.1 ms on 32 members of 64-448^2 cells, 8.0 instead of 6.9 on 100).
+int seg_rows_for(int fixed) { return fixed > 0 ? fixed : 8; }
 
 int cluster_for(const vf_handle* h, const Opts& o) {
   const long long tiles =
@@ -250,6 +262,7 @@ void destroy_batch(vf_batch* b) {
 
 constexpr int kChunk = 16;    // steps per graph launch of a wide member
 constexpr int kInFlight = 3;  // chunks kept queued per wide member (rides out host stalls)
+constexpr int kPlainChunks = 4;  // chunks a handle runs kernel by kernel before its graph is captured
 
 // Final result of a wide member from the record copy of its last retired chunk.
 void wide_finish(vf_batch* b, Wide& w, const vf::StepRecord& r, long long k, int status) {
@@ -266,11 +279,13 @@ void wide_finish(vf_batch* b, Wide& w, const vf::StepRecord& r, long long k, int
 
 int wide_enqueue(vf_batch* b, Wide& w) {
   vf_handle* h = b->hs[w.member];
-  const long long left = w.max_steps - w.enqueued;
-  const int n = (int)std::min<long long>(kChunk, left);
-  int rc = (n == kChunk && (w.enqueued & 1) == 0) ? vf::handle_enqueue_chunk(h, kChunk)
-                                                  : vf::handle_enqueue_steps(h, w.enqueued, n);
-  if (rc) return rc;
+  // A handle's first chunks are launched kernel by kernel: capturing and
+  // instantiating the graph costs as much host time as a few of them. Graph
+  // chunks are whole: steps past max_steps find their record inactive.
+  const bool graph = (w.enqueued & 1) == 0 && (h->chunk_exec || h->plain_chunks >= kPlainChunks);
+  const int n = graph ? kChunk : (int)std::min<long long>(kChunk, w.max_steps - w.enqueued);
+  h->plain_chunks += graph ? 0 : 1;
+  if (int rc = graph ? vf::handle_enqueue_chunk(h, kChunk) : vf::handle_enqueue_steps(h, w.enqueued, n)) return rc;
   w.enqueued += n;
   const int slot = (w.head + w.inflight) % kInFlight;
   cudaError_t e = cudaMemcpyAsync(slot_rec(b->slots[w.member], slot), h->rec, sizeof(vf::StepRecord),
@@ -302,11 +317,7 @@ int pump(vf_batch* b) {
       if (r.wait_fault)
         return bfail(b, VF_ECUDA, "wide member: a bounded wait for a TMA tile copy gave up");
       if (!r.active[k & 1]) {
-        wide_finish(b, w, r, k, vf::kEnsOk);
-        break;
-      }
-      if (k >= w.max_steps) {
-        wide_finish(b, w, r, k, vf::kEnsMaxSteps);
+        wide_finish(b, w, r, k, r.n_done >= w.max_steps && r.t[k & 1] < w.endtime ? vf::kEnsMaxSteps : vf::kEnsOk);
         break;
       }
       if (r.t[k & 1] == w.last_t && k > 0) {  // a whole chunk without progress
@@ -378,10 +389,11 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
   std::vector<double> work(n);
   for (int i = 0; i < n; ++i) {
     const vf_handle* h = hs[i];
-    if ((long long)h->cfg.nx * h->cfg.ny >= o.wide_cells) {
+    if ((long long)h->cfg.nx * h->cfg.ny >= wide_cells_for(h, o)) {
       Wide w;
       w.member = i;
       w.max_steps = max_steps > 0 ? max_steps : LLONG_MAX;
+      w.endtime = endtime[i];
       w.last_t = t0[i];
       b->wide.push_back(w);
       continue;
@@ -408,7 +420,8 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     vf_handle* h = hs[w.member];
     bool ok = true;
     for (cudaEvent_t& e : w.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-    int rc = ok ? vf::handle_begin_loop(h, t0[w.member], endtime[w.member], match_endtime, maximum_timestep)
+    int rc = ok ? vf::handle_begin_loop(h, t0[w.member], endtime[w.member], match_endtime, maximum_timestep,
+                                           max_steps)
                 : VF_ECUDA;
     for (int k = 0; rc == VF_OK && k < kInFlight && w.enqueued < w.max_steps; ++k) rc = wide_enqueue(b, w);
     if (rc) {
@@ -461,12 +474,12 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
         order.push_back((int)itd.size());
         itd.push_back(make_item<double>(h, h->ad, t0[i], endtime[i], match_endtime, maximum_timestep, max_steps, res,
                                          b->epoch_d));
-        itd.back().seg_rows = seg_rows_for(h, g.csize, o.seg_rows);
+        itd.back().seg_rows = seg_rows_for(o.seg_rows);
       } else {
         order.push_back((int)itf.size());
         itf.push_back(make_item<float>(h, h->af, t0[i], endtime[i], match_endtime, maximum_timestep, max_steps, res,
                                         b->epoch_d));
-        itf.back().seg_rows = seg_rows_for(h, g.csize, o.seg_rows);
+        itf.back().seg_rows = seg_rows_for(o.seg_rows);
       }
     }
   }

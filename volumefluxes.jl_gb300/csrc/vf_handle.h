@@ -38,6 +38,7 @@ struct vf_handle {
   int sample_cap = 0;
   cudaGraphExec_t chunk_exec = nullptr;  // captured chunk of steps (wide batch members)
   int chunk_k = 0;                        // its step count; 0: recapture
+  int plain_chunks = 0;                   // chunks run without a graph so far
   void* chunk_u0 = nullptr;               // U[0] when captured (the buffers swap between calls)
 };
 
@@ -46,9 +47,10 @@ namespace vf {
 // and makes its device current; on failure records the message on h.
 int handle_ready(vf_handle* h);
 // Device-resident time loop of vf_simulate, driven asynchronously: write the
-// loop's record (t0, end time, match_endtime, maximum_timestep < 0: none) to
-// the device on the handle's stream.
-int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep);
+// loop's record (t0, end time, match_endtime, maximum_timestep < 0: none,
+// max_steps <= 0: none) to the device on the handle's stream.
+int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep,
+                      long long max_steps);
 // Copies the step record to the host (h->rec_h) and waits for the stream; an
 // error when a bounded wait of a step gave up.
 int handle_pull_record(vf_handle* h);

@@ -71,6 +71,7 @@ struct StepRecord {
   double stop_time;
   double last_dt;
   long long n_done;
+  long long max_steps;  // device loop: stop after this many steps (0: no limit)
   double explicit_max_dt;
   int explicit_mode;
   int force_dt;        // 1: every step uses forced_dt (a frozen dt sequence)
@@ -536,8 +537,10 @@ __device__ __forceinline__ void advance_record(StepRecord* rec, int parity, doub
   const double tn = next_time<T>(rec->t[parity], dt);
   rec->last_dt = dt;
   rec->t[parity ^ 1] = tn;
-  rec->n_done += 1;
-  const bool more = !rec->explicit_mode && (tn < rec->endtime) && !(tn + dt >= rec->stop_time);
+  const long long done = rec->n_done + 1;
+  rec->n_done = done;
+  const bool more = !rec->explicit_mode && (tn < rec->endtime) && !(tn + dt >= rec->stop_time) &&
+                    !(rec->max_steps > 0 && done >= rec->max_steps);
   rec->active[parity ^ 1] = more ? 1 : 0;
   rec->speed_bits[parity ^ 1][0] = 0ull;
   rec->speed_bits[parity ^ 1][1] = 0ull;

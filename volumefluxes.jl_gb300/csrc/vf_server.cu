@@ -74,7 +74,6 @@ struct vf_server {
   int device = 0;
   size_t budget = 0, used = 0;
   vf_batch_options opt{};
-  bool has_opt = false;
   int64_t max_steps = 0;
   int64_t next_ticket = 1;
   std::deque<int64_t> queue;
@@ -181,7 +180,7 @@ int admit_and_launch(vf_server* s) {
   if (hs.empty()) return VF_OK;
   vf_batch* b = nullptr;
   int rc = vf_batch_launch(hs.data(), (int32_t)hs.size(), t0.data(), ends.data(), 1, -1.0, s->max_steps,
-                           s->has_opt ? &s->opt : nullptr, &b);
+                           &s->opt, &b);
   if (rc) {
     const std::string msg = vf_batch_last_error(nullptr);
     for (int64_t tk : tickets) finish_request(s, s->reqs[tk], rc, msg);
@@ -241,10 +240,11 @@ int vf_server_create(int32_t device, int64_t hbm_budget_bytes, const vf_batch_op
   s->device = device;
   s->budget = (size_t)hbm_budget_bytes;
   s->max_steps = max_steps;
-  if (opt) {
-    s->opt = *opt;
-    s->has_opt = true;
-  }
+  if (opt) s->opt = *opt;
+  // Requests keep clusters up to 512^2 cells by default: the batch's lower
+  // threshold shares the GPU evenly, which answers small requests later while
+  // large ones run.
+  if (s->opt.wide_cells == 0) s->opt.wide_cells = 1 << 18;
   s->t0 = std::chrono::steady_clock::now();
   try {
     s->engine = std::thread(engine_loop, s);
