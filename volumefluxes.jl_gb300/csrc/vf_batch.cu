@@ -173,12 +173,11 @@ long long wide_cells_for(const vf_handle* h, const Opts& o) {
   return h->elem == 8 ? 8192 : 65536;
 }
 
-// Kernel design of a member, as the plain path chooses it (vf_abi.cu
-// select_variants): column marching for Float32 members with wall BCs, linear
+// Kernel design of a cluster member: column marching for Float32 members with wall BCs, linear
 // reconstruction and constant sources (0 with RK2, 2 with forward Euler);
 // tiles (1) for everything else.
 int variant_of(const vf_handle* h) {
-  if (h->elem == 4 && h->af.variant == 0) return h->af.rk2 ? 0 : 2;
+  if (h->elem == 4 && h->af.variant == 0 && !h->af.general) return h->af.rk2 ? 0 : 2;
   return 1;
 }
 

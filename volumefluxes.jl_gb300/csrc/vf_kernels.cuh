@@ -896,7 +896,9 @@ __global__ void __launch_bounds__(S::NT, S::MINB)
 // ---------------------------------------------------------------------------
 // Forward-Euler apply pass: U1 = clamp((U0 + dt*L) ./ (1 .- dt*[0,S,S])).
 // Forward-Euler apply over one tile at (x0, y0): the pointwise stage-1 update.
-template <typename T, bool CG>
+// NEU: NeumannBC as well, whose isolated ghosts (friction included) would hold
+// every other kernel to a third of its threads: 154 instead of 40 registers.
+template <typename T, bool CG, bool NEU = true>
 __device__ __forceinline__ void apply_fe_tile(const Geom<T>& g, const Phys<T>& p, const T* U0,
                                               const T* __restrict__ B, const T* Lin, const T* Sin, T* Uo, int x0,
                                               int y0, double dt, double t) {
@@ -916,7 +918,7 @@ __device__ __forceinline__ void apply_fe_tile(const Geom<T>& g, const Phys<T>& p
     stage1_point<T>(p, tdt, gld<CG>(U0 + o), gld<CG>(U0 + g.PS + o), gld<CG>(U0 + 2 * g.PS + o), gld<CG>(Lin + o),
                     gld<CG>(Lin + g.PS + o), gld<CG>(Lin + 2 * g.PS + o), S, Bc, w, hu, hv);
     store_with_ghosts<T>(g, Uo, gx, gy, w, hu, hv);
-    if (g.bc == 3 && (gx == g.gc + g.nx - 1 || gy == g.gc + g.ny - 1)) {
+    if (NEU && g.bc == 3 && (gx == g.gc + g.nx - 1 || gy == g.gc + g.ny - 1)) {
       T scal[8];
       if (p.any_dynamic) point_scalars<T>(p, t, scal);
       if (gx == g.gc + g.nx - 1) neumann_outer<T, CG>(g, p, tdt, U0, B, scal, g.N1 - 1, gy, 0, false, Uo);
@@ -925,7 +927,7 @@ __device__ __forceinline__ void apply_fe_tile(const Geom<T>& g, const Phys<T>& p
   }
 }
 
-template <typename T>
+template <typename T, bool NEU>
 __global__ void __launch_bounds__(NT) k_apply_fe(Geom<T> g, Phys<T> p, const T* __restrict__ U0,
                                                  const T* __restrict__ B, const T* __restrict__ Lin,
                                                  const T* __restrict__ Sin, T* __restrict__ Uo, StepRecord* rec,
@@ -939,7 +941,7 @@ __global__ void __launch_bounds__(NT) k_apply_fe(Geom<T> g, Phys<T> p, const T* 
   if (threadIdx.x == 0) sdt = step_dt<T>(g, rec, parity);
   __syncthreads();
   const double dt = sdt;
-  apply_fe_tile<T, false>(g, p, U0, B, Lin, Sin, Uo, g.gc + blockIdx.x * TX, g.gc + blockIdx.y * TY, dt,
+  apply_fe_tile<T, false, NEU>(g, p, U0, B, Lin, Sin, Uo, g.gc + blockIdx.x * TX, g.gc + blockIdx.y * TY, dt,
                           rec->t[parity]);
   if (root) advance_record<T>(rec, parity, dt);
 }

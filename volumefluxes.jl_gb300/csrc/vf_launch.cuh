@@ -22,6 +22,7 @@ struct StepArgs {
   Phys<T> p;
   int rk2;
   int variant;  // 0: column-marching kernels, 1: shared-memory tile kernels
+  int general;  // marching: the kernels for every boundary kind, reconstruction and source (Float32)
   const T* B;
   T* L;
   T* S;

@@ -132,13 +132,16 @@ __device__ __forceinline__ Cell3<T> load_cell(const Geom<T>& g, const T* U, int 
   return c;
 }
 
-// Reconstruction of this lane's cell along y (DIR 1) or x (DIR 0).
-template <typename T>
-__device__ __forceinline__ void recon(const Phys<T>& p, const Cell3<T>& l, const Cell3<T>& c, const Cell3<T>& r, T Bl,
-                                      T Br, Cell3<T>& L, Cell3<T>& R) {
+// Reconstruction of this lane's cell along y (DIR 1) or x (DIR 0); lo and hi are
+// the cell's corner rows.
+template <typename T, bool GEN>
+__device__ __forceinline__ void recon(const Geom<T>& g, const Phys<T>& p, const Cell3<T>& l, const Cell3<T>& c,
+                                      const Cell3<T>& r, T Bl, T Br, const CornerRow<T>& lo, const CornerRow<T>& hi,
+                                      Cell3<T>& L, Cell3<T>& R) {
   const T lv[3] = {l.w, l.hu, l.hv}, cv[3] = {c.w, c.hu, c.hv}, rv[3] = {r.w, r.hu, r.hv};
   T Lv[3], Rv[3];
-  reconstruct_cell<T>(p, lv, cv, rv, Bl, Br, Lv, Rv);
+  if (GEN && p.rec_none) no_reconstruction<T>(cv, b_cell(g, lo, hi), Lv, Rv);
+  else reconstruct_cell<T>(p, lv, cv, rv, Bl, Br, Lv, Rv);
   L = Cell3<T>{Lv[0], Lv[1], Lv[2]};
   R = Cell3<T>{Rv[0], Rv[1], Rv[2]};
 }
@@ -168,7 +171,7 @@ __device__ __forceinline__ T add_bottom(const Phys<T>& p, T acc, T slope, T hmea
 // plus the bottom source along x (src/numericalflux/numericalflux.jl:24-30,
 // src/sourceterms/source_term_bottom.jl:34-40). Every lane participates in the
 // shuffles; lanes 2..30 compute valid faces x-1/2.
-template <typename T, bool SPEED, bool SEL>
+template <typename T, bool SPEED, bool SEL, bool GEN>
 __device__ __forceinline__ Cell3<T> x_derivative(const Geom<T>& g, const Phys<T>& p, const Cell3<T>& u,
                                                  const CornerRow<T>& clo, const CornerRow<T>& chi, T& sx) {
   Cell3<T> ul{shfl_up1(u.w), shfl_up1(u.hu), shfl_up1(u.hv)};
@@ -176,7 +179,7 @@ __device__ __forceinline__ Cell3<T> x_derivative(const Geom<T>& g, const Phys<T>
   const T bl = b_xface_l(g, clo, chi);
   const T br = shfl_dn1(bl);  // right x-face of x == left x-face of x+1
   Cell3<T> L, R;
-  recon<T>(p, ul, u, ur, bl, br, L, R);
+  recon<T, GEN>(g, p, ul, u, ur, bl, br, clo, chi, L, R);
   const Cell3<T> Rm{shfl_up1(R.w), shfl_up1(R.hu), shfl_up1(R.hv)};
   T sp = (T)0;
   const Cell3<T> Fl = face<T, 0, SPEED, SEL>(p, Rm, L, sp);  // face x-1/2
@@ -224,12 +227,23 @@ __device__ __forceinline__ void block_speed_commit(StepRecord* rec, int parity, 
 }
 
 // ---------------------------------------------------------------------------
+// Rain and infiltration of an output cell (GEN: the time- and cell-dependent ones too).
+template <typename T, bool GEN>
+__device__ __forceinline__ T march_sources(const Geom<T>& g, const Phys<T>& p, T acc, const T* scal, const StripGeom& s,
+                                           int j) {
+  if constexpr (GEN) {
+    if (p.any_dynamic) return s.out_col ? add_point_sources<T>(p, acc, scal, sidx(g, s.x, j)) : acc;
+  }
+  return add_point_sources<T>(p, acc);
+}
+
 // Flux pass of one strip segment (warp-collective): L(U0), S(U0); mx, my
-// collect the warp's CFL maxima as bit-pattern keys.
-template <typename T, bool CG>
+// collect the warp's CFL maxima as bit-pattern keys. scal holds point_scalars().
+template <typename T, bool CG, bool GEN = false>
 __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>& p, const T* U,
                                                 const T* __restrict__ B, T* Lout, T* Sout, const StripGeom& s,
-                                                unsigned long long& mx_out, unsigned long long& my_out) {
+                                                unsigned long long& mx_out, unsigned long long& my_out,
+                                                const T* scal = nullptr) {
   // Float32 speed keys fit 32 bits: one 32-bit max per face instead of a
   // 64-bit one (the flux pass measured 0.367 instead of 0.385 ms at 4096^2).
   using Key = typename std::conditional<sizeof(T) == 4, unsigned, unsigned long long>::type;
@@ -247,8 +261,8 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
   {
     Cell3<T> Lm, Rm, L0, R0;
     const T blm = b_yface(g, cm1), b0 = b_yface(g, c0), b1 = b_yface(g, c1);
-    recon<T>(p, um2, um1, uc, blm, b0, Lm, Rm);  // row ys-1
-    recon<T>(p, um1, uc, un, b0, b1, L0, R0);    // row ys
+    recon<T, GEN>(g, p, um2, um1, uc, blm, b0, cm1, c0, Lm, Rm);  // row ys-1
+    recon<T, GEN>(g, p, um1, uc, un, b0, b1, c0, c1, L0, R0);     // row ys
     T sp = (T)0;
     y.Gm = face<T, 1, true, kFluxSel>(p, Rm, L0, sp);
     if (s.out_col) my = max(my, (Key)speed_key<T>(sp));
@@ -261,12 +275,12 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
     const Cell3<T> u2 = load_cell<T, CG>(g, U, x, j + 2, s.ld_col);
     const CornerRow<T> c2 = load_corner_row(g, B, x, j + 2);
     T sx = (T)0;
-    Cell3<T> acc = x_derivative<T, true, kFluxSel>(g, p, uc, c0, c1, sx);
+    Cell3<T> acc = x_derivative<T, true, kFluxSel, GEN>(g, p, uc, c0, c1, sx);
     if (s.lane >= 2 && s.lane <= 2 + MOUT && s.x <= g.gc + g.nx) mx = max(mx, (Key)speed_key<T>(sx));
     // y: reconstruct row j+1, flux through face j+1/2
     Cell3<T> Ln, Rn;
     const T b2 = b_yface(g, c2);
-    recon<T>(p, uc, un, u2, y.Br, b2, Ln, Rn);
+    recon<T, GEN>(g, p, uc, un, u2, y.Br, b2, c1, c2, Ln, Rn);
     T sp = (T)0;
     const Cell3<T> Gp = face<T, 1, true, kFluxSel>(p, y.R, Ln, sp);
     if (s.out_col) my = max(my, (Key)speed_key<T>(sp));
@@ -274,7 +288,7 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
     acc.hu = acc.hu - p.inv_dy * (Gp.hu - y.Gm.hu);
     acc.hv = acc.hv - p.inv_dy * (Gp.hv - y.Gm.hv);
     acc.hv = add_bottom<T>(p, acc.hv, slope_over<T>(y.Br - y.Bl, p.dy, p.inv_dy, p.dy_pow2), (y.R.w + y.Lh) * (T)0.5);
-    acc.w = add_point_sources<T>(p, acc.w);
+    acc.w = march_sources<T, GEN>(g, p, acc.w, scal, s, j);
     if (s.out_col) {
       const long long o = sidx(g, x, j);
       Lout[o] = acc.w;
@@ -315,17 +329,27 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
 #ifndef VF_MARCH_FLUX_BLOCKS_F32
 #define VF_MARCH_FLUX_BLOCKS_F32 7
 #endif
-template <typename T> struct MarchStageBlocks { static constexpr int value = sizeof(T) == 4 ? VF_MARCH_STAGE_BLOCKS_F32 : 1; };
+template <typename T> struct MarchStageBlocks {
+  static constexpr int value = sizeof(T) == 4 ? VF_MARCH_STAGE_BLOCKS_F32 : 1;
+  static constexpr int general = sizeof(T) == 4 ? 6 : 1;
+};
 template <typename T> struct MarchFluxBlocks { static constexpr int value = sizeof(T) == 4 ? VF_MARCH_FLUX_BLOCKS_F32 : 1; };
 
-template <typename T>
+// GEN: NoReconstruction and time- or cell-dependent sources as well (the ghost
+// cells come from memory, so the boundary kind does not matter here).
+template <typename T, bool GEN>
 __global__ void __launch_bounds__(MW * MWPB, MarchFluxBlocks<T>::value) k_flux_march(Geom<T> g, Phys<T> p, const T* __restrict__ U,
                                                           const T* __restrict__ B, T* __restrict__ Lout,
                                                           T* __restrict__ Sout, StepRecord* rec, int parity, int seg_rows) {
   if (!rec->active[parity]) return;
+  __shared__ T scal[8];
+  if (GEN && p.any_dynamic) {
+    if (threadIdx.x == 0) point_scalars<T>(p, rec->t[parity], scal);
+    __syncthreads();
+  }
   StripGeom s;
   unsigned long long mx = 0ull, my = 0ull;  // CFL maxima as bit patterns (speeds are >= 0)
-  if (strip_setup(g, seg_rows, s)) flux_march_unit<T, false>(g, p, U, B, Lout, Sout, s, mx, my);
+  if (strip_setup(g, seg_rows, s)) flux_march_unit<T, false, GEN>(g, p, U, B, Lout, Sout, s, mx, my, scal);
   block_speed_commit(rec, parity, mx, my);
 }
 
@@ -345,6 +369,34 @@ __device__ __forceinline__ Cell3<T> stage1_row(const Geom<T>& g, const Phys<T>& 
                     gld<CG>(Lin + 2 * g.PS + o), S, b_cell(g, clo, chi), u1.w, u1.hu, u1.hv);
   }
   return u1;
+}
+
+// The same for any cell of the volume (GEN): ghost cells take U1 of their boundary
+// source cell, computed the same pointwise way from global memory, or for
+// NeumannBC's right and top ghosts their own isolated update; corner ghosts stay
+// zero.
+template <typename T, bool CG>
+__device__ __forceinline__ Cell3<T> stage1_any(const Geom<T>& g, const Phys<T>& p, T tdt, const T* U0, const T* Lin,
+                                               const T* Sin, const T* __restrict__ B, const T* scal, int x, int r,
+                                               bool xin, const CornerRow<T>& clo, const CornerRow<T>& chi,
+                                               Cell3<T>& u0out) {
+  const bool yin = r >= g.gc && r < g.gc + g.ny;
+  if (yin == xin || x >= g.N1 || r >= g.N2) return stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, r, xin, clo, chi, u0out);
+  u0out = Cell3<T>{(T)0, (T)0, (T)0};
+  Cell3<T> u;
+  const int axis = yin ? 0 : 1, v = yin ? x : r, n = yin ? g.nx : g.ny;
+  if (g.bc == 3 && v >= g.gc + n) {
+    T a0, a1, a2, lpt, Bg;
+    neumann_u1<T, CG>(g, p, tdt, U0, B, scal, yin ? g.N1 - 1 : x, yin ? r : g.N2 - 1, u.w, u.hu, u.hv, a0, a1, a2, lpt, Bg);
+    return u;
+  }
+  const int q = bc_source(v, g.gc, n, g.bc, axis);
+  u1_global<T, CG>(g, p, tdt, U0, Lin, Sin, B, yin ? q : x, yin ? r : q, u.w, u.hu, u.hv);
+  if (g.bc == 1) {
+    if (yin) u.hu = -u.hu;
+    else u.hv = -u.hv;
+  }
+  return u;
 }
 
 // Wall ghost columns of a U1 row (src/bc.jl:92-100): ghost lanes read their
@@ -392,14 +444,21 @@ __device__ __forceinline__ void store_march(const Geom<T>& g, const StripGeom& s
   Uo[2 * g.PS + o] = hv;
 }
 
-// RK2 stage pass of one strip segment (warp-collective): U2 with its ghosts into Uo.
-template <typename T, bool CG>
+// RK2 stage pass of one strip segment (warp-collective): U2 with its ghosts into
+// Uo. GEN: every boundary kind, reconstruction and source; otherwise walls,
+// whose ghosts come from the window by shuffles and row mirrors.
+template <typename T, bool CG, bool GEN = false>
 __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>& p, const T* U0,
                                                  const T* __restrict__ B, const T* Lin, const T* Sin, T* Uo,
-                                                 const StripGeom& s, T tdt) {
+                                                 const StripGeom& s, T tdt, const T* scal = nullptr) {
   const int x = s.x;
   const bool xin = x >= g.gc && x < g.gc + g.nx;
   const int top = g.gc + g.ny;  // first top ghost row
+  // U1 of row r between the corner rows lo and hi
+  auto u1_row = [&](int r, const CornerRow<T>& lo, const CornerRow<T>& hi, Cell3<T>& u0) -> Cell3<T> {
+    if constexpr (GEN) return stage1_any<T, CG>(g, p, tdt, U0, Lin, Sin, B, scal, x, r, xin, lo, hi, u0);
+    else return mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, r, xin, lo, hi, u0), r < top);
+  };
   // prologue: corner rows ys-2..ys+2, U1 rows ys-2..ys+1
   const CornerRow<T> cm2 = load_corner_row(g, B, x, s.ys - 2);
   const CornerRow<T> cm1 = load_corner_row(g, B, x, s.ys - 1);
@@ -407,31 +466,31 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
   CornerRow<T> c1 = load_corner_row(g, B, x, s.ys + 1);
   CornerRow<T> c2 = load_corner_row(g, B, x, s.ys + 2);
   Cell3<T> u0c{(T)0, (T)0, (T)0}, u0n{(T)0, (T)0, (T)0}, dummy;
-  Cell3<T> uc = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys, xin, c0, c1, u0c), true);
+  Cell3<T> uc = u1_row(s.ys, c0, c1, u0c);
   Cell3<T> un;
-  if (s.ys + 1 >= top) {
+  if (!GEN && s.ys + 1 >= top) {
     un = mirror_row(uc);  // top ghost above a one-row segment
   } else {
-    un = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys + 1, xin, c1, c2, u0n), true);
+    un = u1_row(s.ys + 1, c1, c2, u0n);
   }
   Cell3<T> um1, um2;
-  if (s.ys == g.gc) {  // bottom ghosts mirror rows gc, gc+1
+  if (!GEN && s.ys == g.gc) {  // bottom ghosts mirror rows gc, gc+1
     um1 = mirror_row(uc);
     um2 = mirror_row(un);
   } else {
-    um1 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys - 1, xin, cm1, c0, dummy), true);
-    if (s.ys == g.gc + 1) um2 = mirror_row(um1);  // one-row segments: the ghost below row gc
-    else um2 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, s.ys - 2, xin, cm2, cm1, dummy), true);
+    um1 = u1_row(s.ys - 1, cm1, c0, dummy);
+    if (!GEN && s.ys == g.gc + 1) um2 = mirror_row(um1);  // one-row segments: the ghost below row gc
+    else um2 = u1_row(s.ys - 2, cm2, cm1, dummy);
   }
   // Ghost row top+1 mirrors row top-2, which leaves the window before it is needed.
   Cell3<T> stash{(T)0, (T)0, (T)0};
-  if (s.ys + 1 == top) stash = mirror_row(um1);
+  if (!GEN && s.ys + 1 == top) stash = mirror_row(um1);
   YCarry<T> y;
   {
     Cell3<T> Lm, Rm, L0, R0;
     const T blm = b_yface(g, cm1), b0 = b_yface(g, c0), b1 = b_yface(g, c1);
-    recon<T>(p, um2, um1, uc, blm, b0, Lm, Rm);
-    recon<T>(p, um1, uc, un, b0, b1, L0, R0);
+    recon<T, GEN>(g, p, um2, um1, uc, blm, b0, cm1, c0, Lm, Rm);
+    recon<T, GEN>(g, p, um1, uc, un, b0, b1, c0, c1, L0, R0);
     T sp;
     y.Gm = face<T, 1, false, kStageSel>(p, Rm, L0, sp);
     y.R = R0;
@@ -443,26 +502,26 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
     // U1 of row j+2 (needs corner rows j+2, j+3)
     const CornerRow<T> c3 = load_corner_row(g, B, x, j + 3);
     Cell3<T> u2, u0x{(T)0, (T)0, (T)0};
-    if (j + 2 == top) {
+    if (!GEN && j + 2 == top) {
       u2 = mirror_row(un);     // row top mirrors top-1
       stash = mirror_row(uc);  // row top+1 mirrors top-2
-    } else if (j + 2 == top + 1) {
+    } else if (!GEN && j + 2 == top + 1) {
       u2 = stash;
     } else {
-      u2 = mirror_columns(g, s, stage1_row<T, CG>(g, p, tdt, U0, Lin, Sin, x, j + 2, xin, c2, c3, u0x), j + 2 < top);
+      u2 = u1_row(j + 2, c2, c3, u0x);
     }
     T sx;
-    Cell3<T> acc = x_derivative<T, false, kStageSel>(g, p, uc, c0, c1, sx);
+    Cell3<T> acc = x_derivative<T, false, kStageSel, GEN>(g, p, uc, c0, c1, sx);
     Cell3<T> Ln, Rn;
     const T b2 = b_yface(g, c2);
-    recon<T>(p, uc, un, u2, y.Br, b2, Ln, Rn);
+    recon<T, GEN>(g, p, uc, un, u2, y.Br, b2, c1, c2, Ln, Rn);
     T sp;
     const Cell3<T> Gp = face<T, 1, false, kStageSel>(p, y.R, Ln, sp);
     acc.w = acc.w - p.inv_dy * (Gp.w - y.Gm.w);
     acc.hu = acc.hu - p.inv_dy * (Gp.hu - y.Gm.hu);
     acc.hv = acc.hv - p.inv_dy * (Gp.hv - y.Gm.hv);
     acc.hv = add_bottom<T>(p, acc.hv, slope_over<T>(y.Br - y.Bl, p.dy, p.inv_dy, p.dy_pow2), (y.R.w + y.Lh) * (T)0.5);
-    acc.w = add_point_sources<T>(p, acc.w);
+    acc.w = march_sources<T, GEN>(g, p, acc.w, scal, s, j);
     if (s.out_col) {
       T w = uc.w + tdt * acc.w;
       T hu = uc.hu + tdt * acc.hu;
@@ -475,6 +534,10 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
         apply_friction<T>(tdt, friction_factor<T>(p, uc.w, uc.hu, uc.hv, Bc), hu, hv);
       dry_clamp<T>(p, w, hu, hv, Bc);
       store_march<T>(g, s, Uo, x, j, w, hu, hv);
+      if (GEN && g.bc == 3) {
+        if (x == g.gc + g.nx - 1) neumann_outer<T, CG>(g, p, tdt, U0, B, scal, g.N1 - 1, j, 0, true, Uo);
+        if (j == g.gc + g.ny - 1) neumann_outer<T, CG>(g, p, tdt, U0, B, scal, x, g.N2 - 1, 1, true, Uo);
+      }
     }
     uc = un;
     un = u2;
@@ -491,8 +554,8 @@ __device__ __forceinline__ void stage_march_unit(const Geom<T>& g, const Phys<T>
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(MW * MWPB, MarchStageBlocks<T>::value) k_stage_march(Geom<T> g, Phys<T> p, const T* __restrict__ U0,
+template <typename T, bool GEN>
+__global__ void __launch_bounds__(MW * MWPB, GEN ? MarchStageBlocks<T>::general : MarchStageBlocks<T>::value) k_stage_march(Geom<T> g, Phys<T> p, const T* __restrict__ U0,
                                                            const T* __restrict__ B, const T* __restrict__ Lin,
                                                            const T* __restrict__ Sin, T* __restrict__ Uo,
                                                            StepRecord* rec, int parity, int seg_rows) {
@@ -502,11 +565,15 @@ __global__ void __launch_bounds__(MW * MWPB, MarchStageBlocks<T>::value) k_stage
     return;
   }
   __shared__ double s_dt;
-  if (threadIdx.x == 0) s_dt = step_dt<T>(g, rec, parity);
+  __shared__ T scal[8];
+  if (threadIdx.x == 0) {
+    s_dt = step_dt<T>(g, rec, parity);
+    if (GEN && p.any_dynamic) point_scalars<T>(p, rec->t[parity], scal);
+  }
   __syncthreads();
   const double dt = s_dt;
   StripGeom s;
-  if (strip_setup(g, seg_rows, s)) stage_march_unit<T, false>(g, p, U0, B, Lin, Sin, Uo, s, (T)dt);
+  if (strip_setup(g, seg_rows, s)) stage_march_unit<T, false, GEN>(g, p, U0, B, Lin, Sin, Uo, s, (T)dt, scal);
   if (root) advance_record<T>(rec, parity, dt);
 }
 

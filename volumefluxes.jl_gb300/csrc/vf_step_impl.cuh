@@ -166,7 +166,9 @@ template <typename T>
 cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cudaStream_t st) {
   if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::flux);
-    k_flux_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
+    const int nb = march_blocks(a.g, seg);
+    if (a.general) k_flux_march<T, true><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
+    else k_flux_march<T, false><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
     return cudaGetLastError();
   }
   if constexpr (sizeof(T) == 8) {
@@ -184,13 +186,17 @@ cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cud
 template <typename T>
 cudaError_t launch_stage_impl(const StepArgs<T>& a, const T* Uin, T* Uout, int parity, cudaStream_t st) {
   if (!a.rk2) {
-    k_apply_fe<T><<<tile_grid<BigTile>(a.g), NT, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    if (a.g.bc == 3)
+      k_apply_fe<T, true><<<tile_grid<BigTile>(a.g), NT, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
+    else
+      k_apply_fe<T, false><<<tile_grid<BigTile>(a.g), NT, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity);
     return cudaGetLastError();
   }
   if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::stage);
-    k_stage_march<T><<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity,
-                                                                    seg);
+    const int nb = march_blocks(a.g, seg);
+    if (a.general) k_stage_march<T, true><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
+    else k_stage_march<T, false><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
     return cudaGetLastError();
   }
   if constexpr (sizeof(T) == 8) {
