@@ -189,6 +189,7 @@ void fill_phys(const vf_handle* h, vf::Phys<T>& p) {
   for (int n = 0; n < p.n_point; ++n) sum += (double)p.point_add[n];
   p.point_sum = (T)sum;
   p.bottom_g = (T)(p.n_bottom * -c.g);
+  p.half_over_kappa = (T)0.5 / p.kappa;
 }
 
 // cuTensorMapEncodeTiled from the driver, looked up once through the runtime

@@ -169,6 +169,7 @@ Opts resolve(const vf_batch_options* o) {
 //   11.3; 100, 24 steps: 9.9 / 6.6 / 6.7; 128 of 64-1024^2, 40 steps: 30.5 /
 //   28.6 / 29.2 (131072 cells: 7.0, 8.2, -, 28.9).
 long long wide_cells_for(const vf_handle* h, const Opts& o) {
+  if (h->elem == 4 && !vf::plane_fits_u32(h->af.g)) return 1;  // the clusters' offsets are 32-bit
   if (o.wide_cells > 0) return o.wide_cells;
   return h->elem == 8 ? 8192 : 65536;
 }

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(NT, EnsBlocks<T>::value) k_ensemble(const EnsI
       for (int u = (int)rank * kWarps + warp; u < nunits; u += csize * kWarps) {
         StripGeom s;
         strip_setup_at(g, seg, u % nstrips, u / nstrips, s);
-        flux_march_unit<T, true>(g, p, U0, sit.B, sit.L, sit.S, s, mx, my);
+        flux_march_unit<T, true, unsigned>(g, p, U0, sit.B, sit.L, sit.S, s, mx, my);
       }
       block_key_max<NT>(mx, my, red, kx, ky);
     } else {
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(NT, EnsBlocks<T>::value) k_ensemble(const EnsI
       for (int u = (int)rank * kWarps + warp; u < nunits; u += csize * kWarps) {
         StripGeom s;
         strip_setup_at(g, seg, u % nstrips, u / nstrips, s);
-        stage_march_unit<T, true>(g, p, U0, sit.B, sit.L, sit.S, U1, s, (T)dt);
+        stage_march_unit<T, true, unsigned>(g, p, U0, sit.B, sit.L, sit.S, U1, s, (T)dt);
       }
     } else if constexpr (VAR == 2) {
       for (int tile = (int)rank; tile < ntiles; tile += csize)

@@ -99,6 +99,12 @@ __device__ __forceinline__ int bc_source(int v, int gc, int n, int bc, int axis)
   return v < gc ? 2 * gc - 1 - v : 2 * (gc + n) - 1 - v;
 }
 
+// Byte offsets within one state plane, and within the corner array, fit 32 bits.
+template <typename T>
+__host__ __device__ inline bool plane_fits_u32(const Geom<T>& g) {
+  return g.PB * (long long)(g.N2 + 1) * (long long)sizeof(T) < (1ll << 32);
+}
+
 template <typename T>
 __device__ __forceinline__ long long sidx(const Geom<T>& g, int x, int y) {
   return (long long)y * g.P + x + XOFF;

@@ -236,6 +236,7 @@ struct Phys {
   T point_add[8];             // kConstant: +rate/3600 for rain, -rate for infiltration
   T point_sum;                // Float32: the constant point sources' sum (summed in Float64)
   T bottom_g;                 // Float32: n_bottom * (-g), the bottom sources' factor at once
+  T half_over_kappa;          // Float32: 0.5 / kappa
   const T* point_field[8];    // kHorton: factor, kField: rain rate [m/s]; total grid, state layout
   const double* tab_t[8];     // kTable: breakpoints of TimeDependentRain
   const double* tab_r[8];     // kTable: rates/3600 per breakpoint
@@ -368,16 +369,9 @@ __device__ __forceinline__ T add_point_sources(const Phys<T>& p, T acc0, const T
 
 // desingularize, src/equations/equation.jl:40-62 (Eq. 26 of Brodtkorb & Holm 2021).
 // For |h| >= kappa the expression equals h exactly: min(...) <= kappa <= |h|.
-// SEL (Float32 only): the same function without a branch, the formula
-// evaluated for every h (|h| >= kappa gives |h| with h's sign, i.e. h), with
-// 1/(2 kappa) as a product; fewer instructions where registers allow.
-template <typename T, bool SEL = false>
+template <typename T>
 __device__ __forceinline__ T desing(T h, T kappa) {
   using A = Arith<T>;
-  if constexpr (SEL && sizeof(T) == 4) {
-    const float m = fminf(h * h * (0.5f / kappa) + kappa * 0.5f, kappa);
-    return copysignf(fmaxf(fabsf(h), m), h);
-  }
   if (!A::abs_lt(h, kappa)) return h;
   const T m = A::min(A::div(h * h, (T)2 * kappa) + kappa / (T)2, kappa);
   return copysign((T)1, h) * A::max(fabs(h), m);
@@ -416,10 +410,10 @@ __device__ __forceinline__ void velocities(const Phys<T>& p, T h, T hs, T hu, T 
 
 // One side of a face: physical flux (src/equations/swe_2D.jl:43-65) and the
 // two outer eigenvalues (src/equations/swe_2D.jl:69-81).
-template <typename T, int DIR, bool SEL = false>
+template <typename T, int DIR>
 __device__ __forceinline__ void side_flux(const Phys<T>& p, T h, T hu, T hv, T& f0, T& f1, T& f2, T& l1, T& l2) {
   using A = Arith<T>;
-  const T hs = desing<T, SEL>(h, p.kappa);
+  const T hs = desing<T>(h, p.kappa);
   T u, v;
   velocities<T>(p, h, hs, hu, hv, u, v);
   T rh = h;
@@ -444,16 +438,83 @@ __device__ __forceinline__ void side_flux(const Phys<T>& p, T h, T hu, T hv, T& 
   l2 = un - c;
 }
 
+// One side of a Float32 face without branches: a dry side takes depth and
+// reciprocal depth zero, so its flux and eigenvalues come out as zeros. wet: the
+// side's depth exceeds the cutoff.
+template <int DIR>
+__device__ __forceinline__ void side_flux_f32(const Phys<float>& p, bool wet, float h, float u, float v,
+                                              float& f0, float& f1, float& f2, float& l1, float& l2) {
+  const float hz = wet ? h : 0.f;
+  const float rh = p.rho * hz;
+  const float hh = hz * hz;
+  const float un = DIR == 0 ? u : v;
+  f0 = rh * un;
+  if (DIR == 0) {
+    f1 = f0 * u + p.c2 * hh;
+    f2 = f0 * v;
+  } else {
+    f1 = (rh * u) * v;
+    f2 = f0 * v + p.c2 * hh;
+  }
+  const float c = sqrtf(p.g * hz);
+  l1 = un + c;
+  l2 = un - c;
+}
+
+// cu_face for Float32. Branches cost the issue-bound marching kernels more than
+// the work they skip: their own instructions, the zeros for the path not taken,
+// and constants loaded anew on each side (the uniform registers are not
+// available to divergent code).
+template <int DIR, bool SPEED>
+__device__ __forceinline__ void cu_face_f32(const Phys<float>& p, float mh, float mhu, float mhv, float ph, float phu,
+                                            float phv, float& F0, float& F1, float& F2, float& speed) {
+  using A = Arith<float>;
+  const bool wm = mh > p.cutoff, wp = ph > p.cutoff;
+  // h* = max(h, min(h^2 / (2 kappa) + kappa/2, kappa)) for h > 0 (src/equations/equation.jl:40-62)
+  const float hm = fmaxf(mh, fminf(mh * mh * p.half_over_kappa + p.kappa * 0.5f, p.kappa));
+  const float hp = fmaxf(ph, fminf(ph * ph * p.half_over_kappa + p.kappa * 0.5f, p.kappa));
+  const float rm = wm ? A::rcp(hm) : 0.f, rp = wp ? A::rcp(hp) : 0.f;
+  float mu = mhu * rm, mv = mhv * rm, pu = phu * rp, pv = phv * rp;
+  const bool nm = wm && mh < p.near_dry, np = wp && ph < p.near_dry;
+  if (nm || np) {  // thin films take the Float64 quotient's bits
+    if (nm) {
+      mu = f64_quotient_f32(mhu, hm);
+      mv = f64_quotient_f32(mhv, hm);
+    }
+    if (np) {
+      pu = f64_quotient_f32(phu, hp);
+      pv = f64_quotient_f32(phv, hp);
+    }
+  }
+  float fm0, fm1, fm2, em1, em2, fp0, fp1, fp2, ep1, ep2;
+  side_flux_f32<DIR>(p, wm, mh, mu, mv, fm0, fm1, fm2, em1, em2);
+  side_flux_f32<DIR>(p, wp, ph, pu, pv, fp0, fp1, fp2, ep1, ep2);
+  const float aplus = fmaxf(fmaxf(ep1, em1), 0.f);
+  const float aminus = fminf(fminf(ep2, em2), 0.f);
+  const float d = aplus - aminus;
+  const bool waves = !(d < p.kappa);
+  const float R = waves ? A::rcp(d) : 0.f;
+  const float q = (aplus * aminus) * R;
+  F0 = (aplus * fm0 - aminus * fp0) * R + q * (ph - mh);
+  F1 = (aplus * fm1 - aminus * fp1) * R + q * (phu - mhu);
+  F2 = (aplus * fm2 - aminus * fp2) * R + q * (phv - mhv);
+  if (SPEED) speed = waves && !(mh < p.cutoff && ph < p.cutoff) ? fmaxf(aplus, -aminus) : 0.f;
+}
+
 // Central-upwind flux across one face, src/numericalflux/swe/centralupwind.jl:48-77.
 // minus = right face value of the left cell, plus = left face value of the right cell.
-template <typename T, int DIR, bool SPEED, bool SEL = false>
+template <typename T, int DIR, bool SPEED>
 __device__ __forceinline__ void cu_face(const Phys<T>& p, T mh, T mhu, T mhv, T ph, T phu, T phv, T& F0, T& F1, T& F2,
                                         T& speed) {
   using A = Arith<T>;
+  if constexpr (std::is_same<T, float>::value) {
+    cu_face_f32<DIR, SPEED>(p, mh, mhu, mhv, ph, phu, phv, F0, F1, F2, speed);
+    return;
+  }
   T fm0 = 0, fm1 = 0, fm2 = 0, em1 = 0, em2 = 0;
-  if (A::gt(mh, p.cutoff)) side_flux<T, DIR, SEL>(p, mh, mhu, mhv, fm0, fm1, fm2, em1, em2);
+  if (A::gt(mh, p.cutoff)) side_flux<T, DIR>(p, mh, mhu, mhv, fm0, fm1, fm2, em1, em2);
   T fp0 = 0, fp1 = 0, fp2 = 0, ep1 = 0, ep2 = 0;
-  if (A::gt(ph, p.cutoff)) side_flux<T, DIR, SEL>(p, ph, phu, phv, fp0, fp1, fp2, ep1, ep2);
+  if (A::gt(ph, p.cutoff)) side_flux<T, DIR>(p, ph, phu, phv, fp0, fp1, fp2, ep1, ep2);
   const T aplus = A::max(A::max(ep1, em1), (T)0);
   const T aminus = A::min(A::min(ep2, em2), (T)0);
   const T d = aplus - aminus;
@@ -590,6 +651,12 @@ __device__ __forceinline__ T friction_factor(const Phys<T>& p, T w, T hu, T hv, 
 template <typename T>
 __device__ __forceinline__ void apply_friction(T tdt, T S, T& hu, T& hv) {
   using A = Arith<T>;
+  if constexpr (sizeof(T) == 4) {  // a select instead of a branch
+    const T f = A::is_zero(S) ? (T)1 : A::rcp((T)1 - tdt * S);
+    hu = hu * f;
+    hv = hv * f;
+    return;
+  }
   if (A::is_zero(S)) return;
   const T den = (T)1 - tdt * S;
   const typename A::Recip R = A::recip(den);

@@ -162,13 +162,33 @@ cudaError_t launch_stage_tiles(const StepArgs<T>& a, const T* Uin, T* Uout, int 
   return cudaGetLastError();
 }
 
+// Calls f(offset type, general form?, bottom kind) with the marching kernels'
+// compile-time form of a handle. 32-bit offsets reach 4 GB of one plane (2^30
+// Float32 cells); larger grids, and Float64, take 64-bit ones.
+template <typename T, typename F>
+void with_march_form(const StepArgs<T>& a, F f) {
+  using u32 = unsigned;
+  using u64 = unsigned long long;
+  const bool small = plane_fits_u32<T>(a.g);
+  if constexpr (sizeof(T) == 8) {
+    if (a.general) f(u64{}, std::true_type{}, std::integral_constant<int, 2>{});
+    else f(u64{}, std::false_type{}, std::integral_constant<int, 2>{});
+  } else {
+    if (!small) f(u64{}, std::true_type{}, std::integral_constant<int, 2>{});
+    else if (a.general) f(u32{}, std::true_type{}, std::integral_constant<int, 2>{});
+    else if (a.g.bottom_const) f(u32{}, std::false_type{}, std::integral_constant<int, 1>{});
+    else f(u32{}, std::false_type{}, std::integral_constant<int, 0>{});
+  }
+}
+
 template <typename T>
 cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cudaStream_t st) {
   if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::flux);
-    const int nb = march_blocks(a.g, seg);
-    if (a.general) k_flux_march<T, true><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
-    else k_flux_march<T, false><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
+    with_march_form(a, [&](auto o, auto gen, auto cb) {
+      k_flux_march<T, decltype(o), decltype(gen)::value, decltype(cb)::value>
+          <<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
+    });
     return cudaGetLastError();
   }
   if constexpr (sizeof(T) == 8) {
@@ -194,9 +214,10 @@ cudaError_t launch_stage_impl(const StepArgs<T>& a, const T* Uin, T* Uout, int p
   }
   if (a.variant == 0) {
     const int seg = march_seg(a.g, MarchSeg<T>::stage);
-    const int nb = march_blocks(a.g, seg);
-    if (a.general) k_stage_march<T, true><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
-    else k_stage_march<T, false><<<nb, MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
+    with_march_form(a, [&](auto o, auto gen, auto cb) {
+      k_stage_march<T, decltype(o), decltype(gen)::value, decltype(cb)::value>
+          <<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
+    });
     return cudaGetLastError();
   }
   if constexpr (sizeof(T) == 8) {
