@@ -185,6 +185,10 @@ void fill_phys(const vf_handle* h, vf::Phys<T>& p) {
       p.any_dynamic = 1;
     }
   }
+  p.n_fields = 0;
+  for (int n = 0; n < 8; ++n) p.field[n] = nullptr;
+  for (int n = 0; n < p.n_point; ++n)
+    if (p.point_kind[n] == vf::kHorton || p.point_kind[n] == vf::kField) p.field[p.n_fields++] = p.point_field[n];
   double sum = 0.0;
   for (int n = 0; n < p.n_point; ++n) sum += (double)p.point_add[n];
   p.point_sum = (T)sum;

@@ -340,7 +340,7 @@ struct SmemFlux {
   T R[S::DIRS * 3 * S::LRN];
   T F[S::DIRS * 3 * S::FN];
   unsigned long long red[2][S::NT / 32];
-  T scal[8];
+  T scal[kScalars];
   unsigned long long bar;  // mbarrier of the tile copies
   int plain;               // 0: staged by TMA; 1: not staged (alignment); 2: the wait gave up
 };
@@ -694,7 +694,7 @@ struct SmemStage {
   T U0[3 * S::TX * S::TY];
   T B[S::BHX * S::BHY];
   double dt;
-  T scal[8];
+  T scal[kScalars];
   unsigned long long bar;  // mbarrier of the tile copies
   int plain;               // 0: staged by TMA; 1: not staged (alignment); 2: the wait gave up
 };
@@ -925,7 +925,7 @@ __device__ __forceinline__ void apply_fe_tile(const Geom<T>& g, const Phys<T>& p
                     gld<CG>(Lin + g.PS + o), gld<CG>(Lin + 2 * g.PS + o), S, Bc, w, hu, hv);
     store_with_ghosts<T>(g, Uo, gx, gy, w, hu, hv);
     if (NEU && g.bc == 3 && (gx == g.gc + g.nx - 1 || gy == g.gc + g.ny - 1)) {
-      T scal[8];
+      T scal[kScalars];
       if (p.any_dynamic) point_scalars<T>(p, t, scal);
       if (gx == g.gc + g.nx - 1) neumann_outer<T, CG>(g, p, tdt, U0, B, scal, g.N1 - 1, gy, 0, false, Uo);
       if (gy == g.gc + g.ny - 1) neumann_outer<T, CG>(g, p, tdt, U0, B, scal, gx, g.N2 - 1, 1, false, Uo);

@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(MW * MWPB, MarchFluxBlocks<T>::value) k_flux_m
                                                           const T* __restrict__ B, T* __restrict__ Lout,
                                                           T* __restrict__ Sout, StepRecord* rec, int parity, int seg_rows) {
   if (!rec->active[parity]) return;
-  __shared__ T scal[8];
+  __shared__ T scal[kScalars];
   if (GEN && p.any_dynamic) {
     if (threadIdx.x == 0) point_scalars<T>(p, rec->t[parity], scal);
     __syncthreads();
@@ -590,7 +590,7 @@ __global__ void __launch_bounds__(MW * MWPB, GEN ? MarchStageBlocks<T>::general 
   // dt in the state's type, shared: left to every thread, the conversion from
   // double was redone three times a row, on the FP64 pipe.
   __shared__ T s_dt;
-  __shared__ T scal[8];
+  __shared__ T scal[kScalars];
   double dt = 0.0;
   if (threadIdx.x == 0) {
     dt = step_dt<T>(g, rec, parity);

@@ -238,6 +238,8 @@ struct Phys {
   T bottom_g;                 // Float32: n_bottom * (-g), the bottom sources' factor at once
   T half_over_kappa;          // Float32: 0.5 / kappa
   const T* point_field[8];    // kHorton: factor, kField: rain rate [m/s]; total grid, state layout
+  int n_fields;               // Float32: sources with a field, in order
+  const T* field[8];          // Float32: their fields
   const double* tab_t[8];     // kTable: breakpoints of TimeDependentRain
   const double* tab_r[8];     // kTable: rates/3600 per breakpoint
   int tab_n[8];
@@ -277,22 +279,37 @@ __device__ __forceinline__ double det_exp(double x) {
 // time t (the same t for both RK2 stages, src/system.jl:71-73):
 // TimeDependentRain's tabulated rate (src/sourceterms/source_term_rain.jl:45-54)
 // and Horton's fc + (f0 - fc)*exp(-k*t) (src/sourceterms/source_term_infiltration.jl:68-70).
+// Float64: one scalar per source, added in list order. Float32: the sum of all
+// that are the same in every cell (summed in Float64) in out[0], then one factor
+// per source with a field, so a cell adds one scalar and its fields.
+constexpr int kScalars = 9;
 template <typename T>
 __device__ __forceinline__ void point_scalars(const Phys<T>& p, double t, T* out) {
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    out[n] = (T)0;
-    if (n >= p.n_point) continue;
-    if (p.point_kind[n] == kTable) {
+  double sum = 0.0;
+  int field = 1;
+#pragma unroll 1
+  for (int n = 0; n < p.n_point; ++n) {
+    double rate = 0.0;
+    if (sizeof(T) == 8) out[n] = (T)0;
+    if (p.point_kind[n] == kConstant) {
+      rate = (double)p.point_add[n];
+    } else if (p.point_kind[n] == kTable) {
       int idx = 0;
       while (idx + 1 < p.tab_n[n] && !(t < p.tab_t[n][idx + 1])) ++idx;
-      out[n] = (T)p.tab_r[n][idx];
+      rate = p.tab_r[n][idx];
+      if (sizeof(T) == 8) out[n] = (T)rate;
     } else if (p.point_kind[n] == kHorton) {
       const T fc = (T)p.horton[n][0], f0 = (T)p.horton[n][1], k = (T)p.horton[n][2];
       const T decay = (T)det_exp((double)(-k * (T)t));
-      out[n] = fc + (f0 - fc) * decay;
+      const T f = fc + (f0 - fc) * decay;
+      if (sizeof(T) == 8) out[n] = f;
+      else out[field++] = -f;
+    } else if (sizeof(T) == 4) {
+      out[field++] = (T)1;
     }
+    sum += rate;
   }
+  if (sizeof(T) == 4) out[0] = (T)sum;
 }
 
 // ΔB/Δ of the bottom source; exact reciprocal multiply when Δ is a power of two.
@@ -354,6 +371,13 @@ __device__ __forceinline__ T add_point_sources(const Phys<T>& p, T acc0) {
 }
 template <typename T>
 __device__ __forceinline__ T add_point_sources(const Phys<T>& p, T acc0, const T* scal, long long cell) {
+  if constexpr (sizeof(T) == 4) {
+    // scal[0]: every source that is the same in all cells; then the fields' factors
+    acc0 = acc0 + scal[0];
+#pragma unroll 1
+    for (int n = 0; n < p.n_fields; ++n) acc0 = acc0 + p.field[n][cell] * scal[1 + n];
+    return acc0;
+  }
 #pragma unroll
   for (int n = 0; n < 8; ++n) {
     if (n >= p.n_point) continue;
