@@ -16,6 +16,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <vector>
 
 #include "vf_handle.h"
 
@@ -55,6 +56,42 @@ cudaMemPool_t device_pool(int device) {
 }  // namespace vf
 
 namespace {
+
+// Host copies of the step record, in pinned memory so that the copies to and from
+// the device run on the stream without staging: slabs of 1024 records kept for
+// the life of the process, handed out and taken back under a lock (freeing pinned
+// memory would synchronise the device).
+std::mutex g_rec_mu;
+std::vector<vf::StepRecord*> g_rec_free;
+
+vf::StepRecord* acquire_record() {
+  std::lock_guard<std::mutex> lk(g_rec_mu);
+  if (g_rec_free.empty()) {
+    constexpr int n = 1024;
+    void* p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(vf::StepRecord) * n, cudaHostAllocPortable) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    try {
+      g_rec_free.reserve(g_rec_free.capacity() + n);
+    } catch (...) {
+      cudaFreeHost(p);
+      return nullptr;
+    }
+    for (int i = n - 1; i >= 0; --i) g_rec_free.push_back(static_cast<vf::StepRecord*>(p) + i);
+  }
+  vf::StepRecord* r = g_rec_free.back();
+  g_rec_free.pop_back();
+  std::memset(r, 0, sizeof(*r));
+  return r;
+}
+
+void release_record(vf::StepRecord* r) {
+  if (!r) return;
+  std::lock_guard<std::mutex> lk(g_rec_mu);
+  g_rec_free.push_back(r);  // never grows past what acquire_record reserved
+}
 
 // Stream-ordered allocation from the library pool on the handle's stream.
 bool dalloc(vf_handle* h, void** p, size_t bytes) {
@@ -411,7 +448,7 @@ void destroy(vf_handle* h) {
     cudaStreamDestroy(h->stream);
   }
   if (h->chunk_exec) cudaGraphExecDestroy(h->chunk_exec);
-  delete h->rec_h;
+  release_record(h->rec_h);
   delete h;
 }
 
@@ -534,7 +571,7 @@ int vf_create(const vf_config* cfg, vf_handle** out) {
   if (cfg->friction != VF_FRICTION_NONE) ok = ok && dalloc(h, &h->S, (size_t)h->PS * h->elem);
   if (!cfg->bottom_is_constant) ok = ok && dalloc(h, &h->B, (size_t)(h->PB * (h->N2 + 1)) * h->elem);
   ok = ok && dalloc(h, reinterpret_cast<void**>(&h->rec), sizeof(vf::StepRecord));
-  h->rec_h = new (std::nothrow) vf::StepRecord();
+  h->rec_h = acquire_record();
   ok = ok && h->rec_h != nullptr;
   h->vol_blocks = 1024;
   ok = ok && dalloc(h, reinterpret_cast<void**>(&h->partial), sizeof(double) * h->vol_blocks);
@@ -751,7 +788,16 @@ int vf_simulate(vf_handle* h, double t0, double endtime, int32_t match_endtime, 
   r->endtime = endtime;
   r->stop_time = stop_time;
   const bool limited = max_steps > 0;
+  r->max_steps = limited ? max_steps : 0;
   if ((rc = push_record(h))) return rc;
+  // Steps are enqueued in chunks, the record is read after each. The first is 8
+  // steps, the others as long as the loop is expected to run at the last dt: steps
+  // past the end cost two empty launches each, a chunk too short a round trip.
+  const double until = std::fmin(endtime, stop_time);
+  auto steps_left = [&](double t, double dt, long long most) -> long long {
+    const double n = dt > 0 ? std::ceil((until - t) / dt) + 1 : 0;
+    return n >= 1 && n < (double)most ? (long long)n : most;
+  };
   long long k = 0;
   long long chunk = 8;
   if (r->active[0]) {
@@ -763,8 +809,7 @@ int vf_simulate(vf_handle* h, double t0, double endtime, int32_t match_endtime, 
       k += n;
       if ((rc = pull_record(h))) return rc;
       if (!h->rec_h->active[k & 1]) break;
-      if (limited && k >= max_steps) break;
-      if (chunk < 256) chunk *= 2;
+      chunk = steps_left(h->rec_h->t[k & 1], h->rec_h->last_dt, 256);
     }
   }
   if (k == 0 && (rc = pull_record(h))) return rc;

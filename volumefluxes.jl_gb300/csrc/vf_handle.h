@@ -20,7 +20,7 @@ struct vf_handle {
   void* S = nullptr;
   void* B = nullptr;
   vf::StepRecord* rec = nullptr;
-  vf::StepRecord* rec_h = nullptr;  // host copy (pageable)
+  vf::StepRecord* rec_h = nullptr;  // host copy (pinned)
   double* partial = nullptr;
   double* vol_out = nullptr;
   void* src_field[VF_MAX_SOURCES] = {};   // per-cell source arrays (state layout)
