@@ -232,7 +232,10 @@ int vf_selftest_near_dry_quotients(int32_t device, const float* a, const float* 
  * concurrent streams), and the GPU's block scheduler starts a pending
  * simulation whenever a cluster finishes. Simulations of at least wide_cells
  * cells instead run the plain whole-grid kernels on their own stream, fed in
- * CUDA-graph chunks by the host whenever the batch is polled or waited on.
+ * CUDA-graph chunks by the host whenever the batch is polled or waited on. With
+ * the default wide_cells, Float64 RK2 simulations of 4096 to 65535 cells are
+ * stepped together, two launches per step for all of them, fed the same way
+ * (fewer than 8 of them: each as a wide one).
  * Per-handle results are bitwise those of vf_simulate on the same handle in
  * Float64, and independent of which other simulations share the batch in both
  * precisions. */

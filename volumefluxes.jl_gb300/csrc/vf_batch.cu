@@ -11,7 +11,10 @@
 // host memory, so the host sees every simulation finish without synchronising
 // the launch it belongs to.
 //
-// Simulations of at least wide_cells interior cells (default 8192 in Float64,
+// Mid-size Float64 simulations are stepped together by launches that span them all
+// (packs below, vf_pack.cuh).
+//
+// Other simulations of at least wide_cells interior cells (default 8192 in Float64,
 // 65536 in Float32; wide_cells_for) are "wide": a 16-CTA cluster would leave most
 // of the GPU to them alone and make them the batch's tail, so they run the plain
 // whole-grid step kernels on their handle's stream instead, as the device loop
@@ -32,6 +35,7 @@
 #include <climits>
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <mutex>
 #include <new>
 #include <string>
@@ -52,12 +56,33 @@ struct Wide {
   double last_t = 0;
   bool done = false;
 };
+// Members stepped together (vf_pack.cuh).
+struct Pack {
+  std::vector<int> members;     // batch indices, in item order
+  std::vector<char> done;
+  std::vector<double> last_t;
+  int live = 0;
+  cudaStream_t stream = nullptr;
+  vf::PackItem<double>* items = nullptr;
+  vf::StepRecord* recs = nullptr;
+  vf::PackBlock* map = nullptr;
+  int n_blocks = 0;
+  int live_at_map = 0;          // members the map holds
+  bool remap = false;           // the map holds a member that must not step again
+  long long enqueued = 0;
+  int head = 0, inflight = 0;   // chunks head .. head+inflight-1; chunk c uses ev/report slot c % 3
+  long long chunk_end[3] = {0, 0, 0};
+  cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
+};
 }  // namespace
 
 struct vf_batch {
   int device = 0;
   int n = 0;
   std::vector<Wide> wide;
+  Pack pack;
+  long long max_steps = 0;         // LLONG_MAX: no limit
+  std::vector<double> endtime;
   std::chrono::steady_clock::time_point start;
   double time_limit_s = 0;
   std::vector<vf_handle*> hs;
@@ -82,8 +107,8 @@ int bfail(vf_batch* b, int code, const std::string& msg) {
 }
 
 // ---- result slots: pinned, device-mapped, never freed ---------------------
-// A slot holds the result a cluster writes (res) and, for wide members, the
-// two step-record copies of the chunks in flight.
+// A slot holds the result a cluster writes (res) and, for wide and packed members,
+// the step-record copies of the chunks in flight.
 struct Slot {
   vf::EnsResult res;
   vf::StepRecord rec[3];
@@ -130,6 +155,7 @@ void release_slots(const std::vector<int>& s) {
 
 vf::EnsResult* slot_host(int s) { return &(g_slabs[s / kSlab] + s % kSlab)->res; }
 vf::EnsResult* slot_dev(int s) { return &(g_slabs_d[s / kSlab] + s % kSlab)->res; }
+vf::StepRecord* slot_rec_dev(int s, int k) { return &(g_slabs_d[s / kSlab] + s % kSlab)->rec[k]; }
 vf::StepRecord* slot_rec(int s, int k) { return &(g_slabs[s / kSlab] + s % kSlab)->rec[k]; }
 
 int slot_done(int s) { return __atomic_load_n(&slot_host(s)->done, __ATOMIC_ACQUIRE); }
@@ -162,9 +188,9 @@ Opts resolve(const vf_batch_options* o) {
 // plain kernels cut a grid into as many blocks as the GPU has room for, where a
 // cluster has 16 CTAs at most; clusters win only while members are small and
 // many. Makespan in ms, all members whole-grid / this threshold / clusters:
-//   Float64, 20 members of 64-224^2, 8 steps: 2.15 / - / 4.0; 8 of 64-160^2:
-//   0.85 / - / 1.75; 200 of 64-256^2, 20 steps: 52 / - / 65; but 200 of
-//   64-80^2, 40 steps: 52 / 42 / 42.
+//   Float64 (before packs, below): 20 members of 64-224^2, 8 steps: 2.15 / - /
+//   4.0; 8 of 64-160^2: 0.85 / - / 1.75; 200 of 64-256^2, 20 steps: 52 / - / 65;
+//   but 200 of 64-80^2, 40 steps: 52 / 42 / 42.
 //   Float32, 16 members of 64-448^2, 60 steps: 4.0 / 4.7 / 10.5; 40: 8.6 / 9.5 /
 //   11.3; 100, 24 steps: 9.9 / 6.6 / 6.7; 128 of 64-1024^2, 40 steps: 30.5 /
 //   28.6 / 29.2 (131072 cells: 7.0, 8.2, -, 28.9).
@@ -172,6 +198,27 @@ long long wide_cells_for(const vf_handle* h, const Opts& o) {
   if (h->elem == 4 && !vf::plane_fits_u32(h->af.g)) return 1;  // the clusters' offsets are 32-bit
   if (o.wide_cells > 0) return o.wide_cells;
   return h->elem == 8 ? 8192 : 65536;
+}
+
+// Float64 RK2 members of kPackCells interior cells and more are stepped together as
+// a pack (vf_pack.cuh) while they are below kAloneCells, where launches of their
+// own, with TMA staging, are 4% faster (24 members of 200-500^2 cells, 24 steps:
+// 29.6 ms packed up to 512^2, 28.4 ms alone); the smallest are left to clusters. A
+// pack takes about 0.1 ms to set up: below kPackMembers of them each goes alone.
+// All designs give the same Float64 bits, so this may depend on the batch.
+// Makespan in ms, pack / all alone / alone from 8192 cells on, clusters below:
+//   20 members of 64-224^2, 8 steps: 1.84 / 2.21 / 4.15; 64: 4.97 / 6.27 / 8.14;
+//   8: 1.12 / 1.09 / 2.17; 4: 0.70 / 0.66 / 1.81; 64 of 64-96^2: 2.53 / 3.75 /
+//   3.79; 200 of 64-80^2, 40 steps: 27.8 / 55.7 / 40.6; 4 of those: 2.17 / 1.66 /
+//   12.3.
+// Forward-Euler and faithful members, and an explicit threshold, are as before.
+constexpr long long kPackCells = 4096, kAloneCells = 65536;
+constexpr int kPackMembers = 8;
+
+bool packs(const vf_handle* h, const Opts& o) {
+  const long long cells = (long long)h->cfg.nx * h->cfg.ny;
+  return o.wide_cells == 0 && cells >= kPackCells && cells < kAloneCells && h->elem == 8 && h->ad.rk2 &&
+         h->ad.variant == 1 && h->ad.arith == VF_ARITH_REFERENCE;
 }
 
 // Kernel design of a cluster member: column marching for Float32 members with wall BCs, linear
@@ -252,6 +299,16 @@ void destroy_batch(vf_batch* b) {
     cudaFreeAsync(b->order_d, b->setup);
     cudaFreeAsync(b->epoch_d, b->setup);
   }
+  Pack& k = b->pack;
+  if (k.stream) {
+    cudaStreamSynchronize(k.stream);
+    if (k.items) cudaFreeAsync(k.items, k.stream);
+    if (k.recs) cudaFreeAsync(k.recs, k.stream);
+    if (k.map) cudaFreeAsync(k.map, k.stream);
+    cudaStreamDestroy(k.stream);
+  }
+  for (cudaEvent_t e : k.ev)
+    if (e) cudaEventDestroy(e);
   for (cudaStream_t s : b->streams) cudaStreamDestroy(s);
   for (Wide& w : b->wide)
     for (cudaEvent_t e : w.ev)
@@ -297,12 +354,162 @@ int wide_enqueue(vf_batch* b, Wide& w) {
   return VF_OK;
 }
 
-// Retire finished chunks of every wide member and keep two in flight.
+// ---- packs ------------------------------------------------------------------
+constexpr int kPackChunk = 8;  // steps per chunk of a pack
+
+// The block map of the pack's live members, uploaded in stream order.
+int pack_map(vf_batch* b, Pack& k) {
+  std::vector<vf::PackBlock> map;
+  for (size_t i = 0; i < k.members.size(); ++i) {
+    if (k.done[i]) continue;
+    const vf_config& c = b->hs[k.members[i]]->cfg;
+    const int n = vf::pack_blocks(c.nx, c.ny);
+    for (int j = 0; j < n; ++j) map.push_back(vf::PackBlock{(int)i, j});
+  }
+  cudaMemPool_t pool = vf::device_pool(b->device);
+  if (k.map) cudaFreeAsync(k.map, k.stream);
+  k.map = nullptr;
+  k.n_blocks = (int)map.size();
+  const size_t bytes = sizeof(vf::PackBlock) * map.size();
+  if (!pool || cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k.map), bytes, pool, k.stream) != cudaSuccess)
+    return VF_ENOMEM;
+  cudaError_t e = cudaMemcpyAsync(k.map, map.data(), bytes, cudaMemcpyHostToDevice, k.stream);
+  // the copy reads a pageable host vector: finish it before the vector goes
+  if (e == cudaSuccess) e = cudaStreamSynchronize(k.stream);
+  k.live_at_map = k.live;
+  k.remap = false;
+  return e == cudaSuccess ? VF_OK : VF_ECUDA;
+}
+
+int pack_enqueue(vf_batch* b, Pack& k) {
+  const int n = (int)std::min<long long>(kPackChunk, b->max_steps - k.enqueued);
+  const vf::PackMap map{k.map, k.n_blocks};
+  const int slot = (k.head + k.inflight) % kInFlight;
+  cudaError_t e = cudaSuccess;
+  for (int i = 0; i < n && e == cudaSuccess; ++i)
+    e = vf::launch_pack_step(k.items, map, (int)((k.enqueued + i) & 1), k.stream);
+  if (e == cudaSuccess) e = vf::launch_pack_report(k.items, (int)k.members.size(), slot, k.stream);
+  if (e == cudaSuccess) e = cudaEventRecord(k.ev[slot], k.stream);
+  if (e != cudaSuccess) return VF_ECUDA;
+  for (size_t j = 0; j < k.members.size(); ++j)
+    if (!k.done[j]) {  // a member that is done may be gone
+      b->hs[k.members[j]]->launches += 2 * n + 1;
+      break;
+    }
+  k.enqueued += n;
+  k.chunk_end[slot] = k.enqueued;
+  k.inflight += 1;
+  return VF_OK;
+}
+
+int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts) {
+  const size_t n = k.members.size();
+  cudaMemPool_t pool = vf::device_pool(b->device);
+  bool ok = pool && cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t& e : k.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+  ok = ok && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k.items), sizeof(vf::PackItem<double>) * n, pool,
+                                     k.stream) == cudaSuccess;
+  ok = ok && cudaMallocFromPoolAsync(reinterpret_cast<void**>(&k.recs), sizeof(vf::StepRecord) * n, pool, k.stream) ==
+                 cudaSuccess;
+  if (!ok) return VF_ENOMEM;
+  std::vector<vf::StepRecord> recs(n);
+  std::vector<vf::PackItem<double>> items(n);
+  for (size_t j = 0; j < n; ++j) {
+    const int i = k.members[j];
+    vf_handle* h = b->hs[i];
+    vf::StepRecord& r = recs[j];
+    std::memset(&r, 0, sizeof(r));
+    r.t[0] = t0[i];
+    r.active[0] = t0[i] < b->endtime[i] ? 1 : 0;
+    r.match_endtime = match ? 1 : 0;
+    r.has_max_ts = max_ts >= 0 ? 1 : 0;
+    r.max_ts = max_ts;
+    r.endtime = b->endtime[i];
+    r.stop_time = std::numeric_limits<double>::infinity();
+    r.max_steps = b->max_steps == LLONG_MAX ? 0 : b->max_steps;
+    vf::PackItem<double>& it = items[j];
+    std::memset(&it, 0, sizeof(it));
+    it.g = h->ad.g;
+    it.p = h->ad.p;
+    it.B = h->ad.B;
+    it.U[0] = static_cast<double*>(h->U[0]);
+    it.U[1] = static_cast<double*>(h->U[1]);
+    it.L = h->ad.L;
+    it.S = h->ad.S;
+    it.rec = k.recs + j;
+    for (int c = 0; c < kInFlight; ++c) it.report[c] = slot_rec_dev(b->slots[i], c);
+  }
+  k.done.assign(n, 0);
+  k.last_t.resize(n);
+  for (size_t j = 0; j < n; ++j) k.last_t[j] = t0[k.members[j]];
+  k.live = (int)n;
+  ok = cudaMemcpyAsync(k.items, items.data(), sizeof(vf::PackItem<double>) * n, cudaMemcpyHostToDevice, k.stream) ==
+       cudaSuccess;
+  ok = ok && cudaMemcpyAsync(k.recs, recs.data(), sizeof(vf::StepRecord) * n, cudaMemcpyHostToDevice, k.stream) ==
+                 cudaSuccess;
+  if (!ok) return VF_ECUDA;
+  if (int rc = pack_map(b, k)) return rc;  // waits for the copies above too
+  for (int c = 0; c < kInFlight && k.enqueued < b->max_steps; ++c)
+    if (int rc = pack_enqueue(b, k)) return rc;
+  return VF_OK;
+}
+
+void pack_finish(vf_batch* b, Pack& k, size_t j, const vf::StepRecord& r, long long end, int status) {
+  vf::EnsResult* res = slot_host(b->slots[k.members[j]]);
+  res->t = r.t[end & 1];
+  res->last_dt = r.last_dt;
+  res->steps = r.n_done;
+  res->status = status;
+  k.done[j] = 1;
+  k.live -= 1;
+  __atomic_store_n(&res->done, 1, __ATOMIC_RELEASE);
+}
+
+// Retires the pack's finished chunks and keeps kInFlight queued.
+int pack_pump(vf_batch* b, Pack& k, bool late) {
+  while (k.inflight > 0) {
+    const int slot = k.head % kInFlight;
+    const cudaError_t q = cudaEventQuery(k.ev[slot]);
+    if (q == cudaErrorNotReady) break;
+    if (q != cudaSuccess) return bfail(b, VF_ECUDA, std::string("pack: ") + cudaGetErrorString(q));
+    const long long end = k.chunk_end[slot];
+    k.head += 1;
+    k.inflight -= 1;
+    for (size_t j = 0; j < k.members.size(); ++j) {
+      if (k.done[j]) continue;
+      const int i = k.members[j];
+      const vf::StepRecord& r = *slot_rec(b->slots[i], slot);
+      const double t = r.t[end & 1];
+      if (!r.active[end & 1])
+        pack_finish(b, k, j, r, end, r.n_done >= b->max_steps && t < b->endtime[i] ? vf::kEnsMaxSteps : vf::kEnsOk);
+      else if (t == k.last_t[j]) {  // a whole chunk without progress
+        // Later chunks still step it: its result is the last one's, and the map
+        // drops it before the next.
+        if (cudaStreamSynchronize(k.stream) != cudaSuccess) return bfail(b, VF_ECUDA, "pack");
+        const int last = k.inflight > 0 ? (k.head + k.inflight - 1) % kInFlight : slot;
+        pack_finish(b, k, j, *slot_rec(b->slots[i], last), k.chunk_end[last], vf::kEnsStalled);
+        k.remap = true;
+      } else if (late && k.inflight == 0)
+        pack_finish(b, k, j, r, end, vf::kEnsTimeout);
+      k.last_t[j] = t;
+    }
+  }
+  if (k.live == 0 || late) return VF_OK;
+  if (k.remap || 2 * k.live <= k.live_at_map)  // half of the members have ended: drop their blocks
+    if (int rc = pack_map(b, k)) return bfail(b, rc, "pack map");
+  while (k.inflight < kInFlight && k.enqueued < b->max_steps)
+    if (int rc = pack_enqueue(b, k)) return bfail(b, rc, "pack launch failed");
+  return VF_OK;
+}
+
+// Retire finished chunks of the pack and of every wide member, keep kInFlight queued.
 int pump(vf_batch* b) {
-  if (b->wide.empty()) return VF_OK;
+  if (b->wide.empty() && b->pack.members.empty()) return VF_OK;
   const double elapsed =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - b->start).count();
   const bool late = elapsed > b->time_limit_s;
+  if (b->pack.live > 0)
+    if (int rc = pack_pump(b, b->pack, late)) return rc;
   for (Wide& w : b->wide) {
     if (w.done) continue;
     while (w.inflight > 0) {
@@ -383,13 +590,21 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
 
   b->start = std::chrono::steady_clock::now();
   b->time_limit_s = o.time_limit_s;
+  b->max_steps = max_steps > 0 ? max_steps : LLONG_MAX;
+  b->endtime.assign(endtime, endtime + n);
   // Wide members apart; the rest in groups by precision, kernel design and
   // cluster size, largest work first inside a group.
   std::vector<Group> groups;
   std::vector<double> work(n);
+  const bool pack = std::count_if(hs, hs + n, [&](const vf_handle* h) { return packs(h, o); }) >= kPackMembers;
   for (int i = 0; i < n; ++i) {
     const vf_handle* h = hs[i];
-    if ((long long)h->cfg.nx * h->cfg.ny >= wide_cells_for(h, o)) {
+    const bool packable = packs(h, o);
+    if (pack && packable) {
+      b->pack.members.push_back(i);
+      continue;
+    }
+    if (packable || (long long)h->cfg.nx * h->cfg.ny >= wide_cells_for(h, o)) {
       Wide w;
       w.member = i;
       w.max_steps = max_steps > 0 ? max_steps : LLONG_MAX;
@@ -414,6 +629,14 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
   for (Group& g : groups)
     std::stable_sort(g.members.begin(), g.members.end(), [&](int a, int c) { return work[a] > work[c]; });
   std::stable_sort(groups.begin(), groups.end(), [](const Group& a, const Group& c) { return a.csize > c.csize; });
+
+  if (pack) {
+    if (int rc = pack_start(b, b->pack, t0, match_endtime, maximum_timestep)) {
+      cudaGetLastError();
+      destroy_batch(b);
+      return bfail(nullptr, rc, "pack start failed");
+    }
+  }
 
   // Wide members start first: their first two chunks go in before any cluster.
   for (Wide& w : b->wide) {
@@ -562,11 +785,16 @@ int vf_batch_collect(vf_batch* b, int32_t i, double* t_out, int64_t* steps_out, 
 int vf_batch_wait(vf_batch* b) {
   if (!b) return bfail(b, VF_EINVAL, "NULL batch");
   if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, VF_ECUDA, "cudaSetDevice failed");
-  for (;;) {  // wide members need the host to feed them
+  for (;;) {  // wide members and packs need the host to feed them
     if (int rc = pump(b)) return rc;
     bool all = true;
     for (const Wide& w : b->wide) all = all && w.done;
+    all = all && b->pack.live == 0;
     if (all) break;
+    if (b->pack.live > 0 && b->pack.inflight > 0) {
+      cudaEventSynchronize(b->pack.ev[b->pack.head % kInFlight]);
+      continue;
+    }
     for (Wide& w : b->wide)
       if (!w.done && w.inflight > 0) {
         cudaEventSynchronize(w.ev[w.head % kInFlight]);

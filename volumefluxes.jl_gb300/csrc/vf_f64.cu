@@ -29,6 +29,23 @@ cudaError_t launch_ensemble(const EnsItem<double>* items, const int* order, int 
 cudaError_t ensemble_max_clusters_f64(int csize, int variant, int* out) {
   return ensemble_max_clusters_impl<double>(csize, variant, out);
 }
+int pack_blocks(int nx, int ny) {
+  Geom<double> g{};
+  g.nx = nx;
+  g.ny = ny;
+  const dim3 t = tile_grid<SmallTile>(g);
+  return (int)(t.x * t.y);
+}
+cudaError_t launch_pack_step(const PackItem<double>* items, const PackMap& m, int parity, cudaStream_t st) {
+  using S = SmallTile;
+  k_pack_flux<double, S><<<m.n, S::NT, sizeof(SmemFlux<double, S>), st>>>(items, m.blocks, parity);
+  k_pack_stage<double, S><<<m.n, S::NT, sizeof(SmemStage<double, S>), st>>>(items, m.blocks, parity);
+  return cudaGetLastError();
+}
+cudaError_t launch_pack_report(const PackItem<double>* items, int n, int slot, cudaStream_t st) {
+  k_pack_report<double><<<(n + 127) / 128, 128, 0, st>>>(items, n, slot);
+  return cudaGetLastError();
+}
 cudaError_t launch_adj_point(const AdjArgs<double>& a, int* nblocks_out, cudaStream_t st) {
   return launch_adj_point_impl<double>(a, nblocks_out, st);
 }

@@ -5,6 +5,7 @@
 #include "vf_adjoint.cuh"
 #include "vf_ensemble.cuh"
 #include "vf_march.cuh"
+#include "vf_pack.cuh"
 
 // Float64 step kernels with faithful quotients and multiply-add contraction
 // (vf_f64f.cu, a unit whose kernels live in their own namespace). `args` points
@@ -53,6 +54,15 @@ cudaError_t launch_ensemble(const EnsItem<double>* items, const int* order, int 
                             unsigned long long time_limit_ns, cudaStream_t st);
 cudaError_t launch_ensemble(const EnsItem<float>* items, const int* order, int n, int csize, int variant,
                             unsigned long long time_limit_ns, cudaStream_t st);
+// A pack (vf_pack.cuh): the blocks of one member, one step of all members, the
+// records' report.
+struct PackMap {
+  const PackBlock* blocks;
+  int n;
+};
+int pack_blocks(int nx, int ny);
+cudaError_t launch_pack_step(const PackItem<double>* items, const PackMap& m, int parity, cudaStream_t st);
+cudaError_t launch_pack_report(const PackItem<double>* items, int n, int slot, cudaStream_t st);
 // Clusters of csize CTAs that fit on the device at once (0: csize not launchable).
 cudaError_t ensemble_max_clusters_f64(int csize, int variant, int* out);
 cudaError_t ensemble_max_clusters_f32(int csize, int variant, int* out);

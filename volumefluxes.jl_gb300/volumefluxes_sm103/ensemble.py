@@ -28,7 +28,8 @@ class BatchOptions:
     smallest power-of-two cluster c <= max_cluster with c * tiles_per_cta >= k;
     Float32 column-marching members split their strips into segments of
     seg_rows rows; members of at least wide_cells cells run the whole-grid
-    kernels instead of a cluster. None keeps the library default. time_limit_s
+    kernels instead of a cluster, and without it mid-size Float64 members are
+    stepped together. None keeps the library default. time_limit_s
     bounds the batch's device time from its start (watchdog)."""
     tiles_per_cta: int | None = None
     max_cluster: int | None = None
