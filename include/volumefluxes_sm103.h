@@ -235,7 +235,8 @@ int vf_selftest_near_dry_quotients(int32_t device, const float* a, const float* 
  * CUDA-graph chunks by the host whenever the batch is polled or waited on. With
  * the default wide_cells, Float64 RK2 simulations of 4096 to 65535 cells are
  * stepped together, two launches per step for all of them, fed the same way
- * (fewer than 8 of them: each as a wide one).
+ * (fewer than 8 of them: each as a wide one), and a host thread of the batch feeds
+ * them between the caller's calls.
  * Per-handle results are bitwise those of vf_simulate on the same handle in
  * Float64, and independent of which other simulations share the batch in both
  * precisions. */

@@ -4,6 +4,7 @@ and just beyond them, with end times of their own, a limit on the steps that is 
 the steps between two reads of the records, and a member whose time stands still.
 Bit for bit the plain loop of every member."""
 import math
+import time
 
 import numpy as np
 import pytest
@@ -80,4 +81,22 @@ def test_a_member_whose_time_stands_still():
     for k in range(1, len(MEMBERS)):
         vf.simulate_to_time(alone[k], ends[k])
         assert res[k].status == N.VF_BATCH_OK and res[k].t == alone[k].t, k
+        assert_same(batch[k], alone[k], k)
+
+
+@pytest.mark.parametrize("members", [3, len(MEMBERS)])  # launches of their own, a pack
+def test_a_batch_left_alone_gets_to_its_end(members):
+    batch, alone = build()[:members], build()[:members]
+    ends = [20 * end for _, end in MEMBERS[:members]]
+    run = E.BatchRun(batch, ends)
+    left, limit = set(range(members)), time.monotonic() + 60
+    while left and time.monotonic() < limit:  # collect does not feed the batch
+        time.sleep(0.05)
+        for i in sorted(left):
+            if run._lib.vf_batch_collect(run._b, i, None, None, None, None) == N.VF_OK:
+                left.remove(i)
+    assert not left
+    for k, r in enumerate(run.finish()):
+        vf.simulate_to_time(alone[k], ends[k])
+        assert r.t == alone[k].t, k
         assert_same(batch[k], alone[k], k)

@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -39,6 +40,7 @@
 #include <mutex>
 #include <new>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "vf_handle.h"
@@ -93,6 +95,11 @@ struct vf_batch {
   int* order_d = nullptr;
   unsigned long long* epoch_d = nullptr;  // watchdog start of the batch
   cudaStream_t setup = nullptr;    // stream of the descriptor copies (streams[0])
+  std::mutex mu;                   // wide, pack and the feeder's error
+  std::thread feeder;
+  int feed_rc = 0;                 // the error that ended the feeder
+  std::string feed_err;
+  std::atomic<bool> stop{false};   // ends the feeder
   std::string err;
 };
 
@@ -100,8 +107,10 @@ namespace {
 
 thread_local std::string g_batch_error;
 
+thread_local bool g_feeding = false;  // this thread is a batch's feeder
+
 int bfail(vf_batch* b, int code, const std::string& msg) {
-  if (b) b->err = msg;
+  if (b) (g_feeding ? b->feed_err : b->err) = msg;
   else g_batch_error = msg;
   return code;
 }
@@ -293,6 +302,8 @@ vf::EnsItem<T> make_item(vf_handle* h, const vf::StepArgs<T>& a, double t0, doub
 
 void destroy_batch(vf_batch* b) {
   if (!b) return;
+  b->stop = true;
+  if (b->feeder.joinable()) b->feeder.join();
   if (b->setup) {
     cudaFreeAsync(b->items_d[0], b->setup);
     cudaFreeAsync(b->items_d[1], b->setup);
@@ -505,6 +516,8 @@ int pack_pump(vf_batch* b, Pack& k, bool late) {
 // Retire finished chunks of the pack and of every wide member, keep kInFlight queued.
 int pump(vf_batch* b) {
   if (b->wide.empty() && b->pack.members.empty()) return VF_OK;
+  std::lock_guard<std::mutex> lk(b->mu);
+  if (b->feed_rc) return bfail(b, b->feed_rc, b->feed_err);
   const double elapsed =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - b->start).count();
   const bool late = elapsed > b->time_limit_s;
@@ -546,6 +559,37 @@ int pump(vf_batch* b) {
       if (int rc = wide_enqueue(b, w)) return bfail(b, rc, "wide member launch: " + b->hs[w.member]->err);
   }
   return VF_OK;
+}
+
+bool fed(const vf_batch* b) {  // nothing left to enqueue
+  return b->pack.live == 0 && std::all_of(b->wide.begin(), b->wide.end(), [](const Wide& w) { return w.done; });
+}
+
+// Feeds the batch while the caller is elsewhere. With the default threshold members
+// that would run to their end in a cluster by themselves depend on the host; a batch
+// that is launched and left alone has to get on all the same. The chunks in flight
+// last several times the interval. An error ends the feeder; the caller's next call
+// returns it.
+void feed(vf_batch* b) {
+  g_feeding = true;
+  if (cudaSetDevice(b->device) != cudaSuccess) return;
+  while (!b->stop) {
+    const int rc = pump(b);
+    {
+      std::lock_guard<std::mutex> lk(b->mu);
+      b->feed_rc = rc;
+      if (rc != VF_OK || fed(b)) return;
+    }
+    std::this_thread::sleep_for(std::chrono::microseconds(100));
+  }
+}
+
+void start_feeder(vf_batch* b) {
+  if (b->wide.empty() && b->pack.members.empty()) return;
+  try {
+    b->feeder = std::thread(feed, b);
+  } catch (...) {  // no thread: the batch is fed when it is polled or waited on
+  }
 }
 
 struct Group {
@@ -656,6 +700,7 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     }
   }
   if (groups.empty()) {
+    if (o.wide_cells == 0) start_feeder(b);
     *out = b;
     return VF_OK;
   }
@@ -747,6 +792,7 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     }
     hs[gr.members.front()]->launches += 1;  // one launch for the whole group
   }
+  if (o.wide_cells == 0) start_feeder(b);
   *out = b;
   return VF_OK;
 }
@@ -787,19 +833,15 @@ int vf_batch_wait(vf_batch* b) {
   if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, VF_ECUDA, "cudaSetDevice failed");
   for (;;) {  // wide members and packs need the host to feed them
     if (int rc = pump(b)) return rc;
-    bool all = true;
-    for (const Wide& w : b->wide) all = all && w.done;
-    all = all && b->pack.live == 0;
-    if (all) break;
-    if (b->pack.live > 0 && b->pack.inflight > 0) {
-      cudaEventSynchronize(b->pack.ev[b->pack.head % kInFlight]);
-      continue;
+    cudaEvent_t next = nullptr;  // the end of the next chunk
+    {
+      std::lock_guard<std::mutex> lk(b->mu);
+      if (fed(b)) break;
+      if (b->pack.live > 0 && b->pack.inflight > 0) next = b->pack.ev[b->pack.head % kInFlight];
+      for (const Wide& w : b->wide)
+        if (!next && !w.done && w.inflight > 0) next = w.ev[w.head % kInFlight];
     }
-    for (Wide& w : b->wide)
-      if (!w.done && w.inflight > 0) {
-        cudaEventSynchronize(w.ev[w.head % kInFlight]);
-        break;
-      }
+    if (next) cudaEventSynchronize(next);
   }
   for (cudaStream_t s : b->streams) {
     cudaError_t e = cudaStreamSynchronize(s);
