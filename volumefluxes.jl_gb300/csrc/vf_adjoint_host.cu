@@ -232,7 +232,7 @@ int backward_impl(vf_adjoint* a, const int32_t* gi, const int32_t* gj, const dou
   VF_ACK(a, cudaMemcpyAsync(a->target, target, sizeof(double) * (size_t)n_g, cudaMemcpyHostToDevice, st));
   VF_ACK(a, cudaMemsetAsync(a->lam, 0, a->state_bytes, st));
   VF_ACK(a, cudaMemsetAsync(a->gB, 0, sizeof(double) * (size_t)(g.N1 + 1) * (g.N2 + 1), st));
-  VF_ACK(a, cudaMemsetAsync(a->gCz_part, 0, sizeof(double) * (size_t)((g.nx + 31) / 32) * ((g.ny + 7) / 8), st));
+  VF_ACK(a, cudaMemsetAsync(a->gCz_part, 0, sizeof(double) * (size_t)vf::adj_point_blocks(g.nx, g.ny), st));
   VF_ACK(a, vf::launch_adj_seed(g, static_cast<const T*>(h->U[0]), static_cast<T*>(a->lam), a->gauges,
                                 a->gauges + n_g, a->target, n_g, a->loss, st));
   VF_ACK(a, cudaStreamSynchronize(st));  // the host vectors above go out of scope
@@ -365,8 +365,7 @@ int vf_adjoint_create(vf_handle* h, int32_t n_steps, int32_t checkpoint_every, v
             alloc(a, &a->C[0], 9 * a->plane_bytes) && alloc(a, &a->C[1], 9 * a->plane_bytes) &&
             alloc(a, &a->gBf[0], 2 * a->plane_bytes) && alloc(a, &a->gBf[1], 2 * a->plane_bytes) &&
             alloc(a, reinterpret_cast<void**>(&a->gB), sizeof(double) * corners) &&
-            alloc(a, reinterpret_cast<void**>(&a->gCz_part), sizeof(double) * (size_t)((h->cfg.nx + 31) / 32) *
-                                                                 ((h->cfg.ny + 7) / 8)) &&
+            alloc(a, reinterpret_cast<void**>(&a->gCz_part), sizeof(double) * (size_t)vf::adj_point_blocks(h->cfg.nx, h->cfg.ny)) &&
             alloc(a, reinterpret_cast<void**>(&a->gCz), sizeof(double)) &&
             alloc(a, reinterpret_cast<void**>(&a->loss), sizeof(double)) &&
             alloc(a, reinterpret_cast<void**>(&a->rec), sizeof(vf::StepRecord)) &&

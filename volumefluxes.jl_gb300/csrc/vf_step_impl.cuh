@@ -258,10 +258,9 @@ cudaError_t launch_volume_impl(const Geom<T>& g, const T* U, const T* B, double*
 
 template <typename T>
 cudaError_t launch_adj_point_impl(const AdjArgs<T>& a, int* nblocks_out, cudaStream_t st) {
-  const dim3 blk(32, 8);
-  const dim3 grid((a.g.nx + 31) / 32, (a.g.ny + 7) / 8);
-  k_adj_point<T><<<grid, blk, 0, st>>>(a);
-  if (nblocks_out) *nblocks_out = (int)(grid.x * grid.y);
+  const int blocks = adj_point_blocks(a.g.nx, a.g.ny);
+  k_adj_point<T><<<blocks, dim3(32, kPointRows), 0, st>>>(a);
+  if (nblocks_out) *nblocks_out = blocks;
   return cudaGetLastError();
 }
 
