@@ -756,7 +756,7 @@ def main():
         sc.w0, sc.hu0, sc.hv0 = d["h"], d["hu"], d["hv"]
     peak, peak_kind = peaks()
     traffic = profile_table("traffic")
-    fp64_inst = profile_table("fp64_inst_per_cell")
+    fp64_inst = profile_table("fp64_pipe_inst_per_cell")
     cells = sc.nx * sc.ny
     dtypes = [args.dtype] + ([] if args.no_variant else [d for d in ("f64", "f32") if d != args.dtype])
     results = {}

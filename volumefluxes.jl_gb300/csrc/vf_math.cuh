@@ -416,7 +416,7 @@ __device__ __forceinline__ float f64_quotient_f32(float a, float b) { return __f
 // Desingularised velocities (hu, hv) / h* (src/equations/equation.jl:40-67).
 // A Float32 state takes the Float64 quotient (f64_quotient_f32) where
 // |h| < p.near_dry, the thin films at wet/dry fronts, and one fast reciprocal
-// elsewhere; Float64 and dual numbers divide in their own type.
+// elsewhere; Float64 divides in its own type.
 template <typename T>
 __device__ __forceinline__ void velocities(const Phys<T>& p, T h, T hs, T hu, T hv, T& u, T& v) {
   using A = Arith<T>;
