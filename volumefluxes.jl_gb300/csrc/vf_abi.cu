@@ -480,7 +480,7 @@ int handle_enqueue_steps(vf_handle* h, long long first, int n) {
 }
 
 int handle_enqueue_chunk(vf_handle* h, int k) {
-  if (!h->chunk_exec || h->chunk_k != k || h->chunk_u0 != h->U[0]) {
+  if (!h->chunk_exec || h->chunk_k != k || h->chunk_u0 != h->U[0] || h->chunk_share != h->af.share) {
     if (h->chunk_exec) {
       cudaGraphExecDestroy(h->chunk_exec);
       h->chunk_exec = nullptr;
@@ -504,6 +504,7 @@ int handle_enqueue_chunk(vf_handle* h, int k) {
     }
     h->chunk_k = k;
     h->chunk_u0 = h->U[0];
+    h->chunk_share = h->af.share;
   }
   VF_CK(h, cudaGraphLaunch(h->chunk_exec, h->stream));
   h->launches += 2LL * k;

@@ -345,6 +345,22 @@ void wide_finish(vf_batch* b, Wide& w, const vf::StepRecord& r, long long k, int
   __atomic_store_n(&res->done, 1, __ATOMIC_RELEASE);
 }
 
+// Wide marching members that take a wave of the GPU together, as a power of two so
+// that chunk graphs are captured anew only when half of them have ended; segment
+// lengths do not change a member's bits, so this may depend on the batch. Four at
+// most: the launches of more do not run side by side often enough. ms at a cap of
+// 1 / 2 / 4 / 8: 16 members of 256-512^2 cells, 60 steps, 6.33 / 5.46 / 5.28 / 6.40;
+// 16 of 128-1024^2 9.11 / 8.77 / 8.93 / 9.10; 32 of 64-448^2, 24 steps, 2.50 / 2.47 /
+// 2.46 / 2.49.
+constexpr int kMarchShare = 4;
+int march_share(const vf_batch* b, const vf_handle* h) {
+  if (h->elem != 4 || h->af.variant != 0) return 0;
+  int live = 0, share = 1;
+  for (const Wide& w : b->wide) live += !w.done && b->hs[w.member]->elem == 4 ? 1 : 0;
+  while (2 * share <= live && share < kMarchShare) share *= 2;
+  return share;
+}
+
 int wide_enqueue(vf_batch* b, Wide& w) {
   vf_handle* h = b->hs[w.member];
   // A handle's first chunks are launched kernel by kernel: capturing and
@@ -353,7 +369,10 @@ int wide_enqueue(vf_batch* b, Wide& w) {
   const bool graph = (w.enqueued & 1) == 0 && (h->chunk_exec || h->plain_chunks >= kPlainChunks);
   const int n = graph ? kChunk : (int)std::min<long long>(kChunk, w.max_steps - w.enqueued);
   h->plain_chunks += graph ? 0 : 1;
-  if (int rc = graph ? vf::handle_enqueue_chunk(h, kChunk) : vf::handle_enqueue_steps(h, w.enqueued, n)) return rc;
+  h->af.share = march_share(b, h);
+  const int rc = graph ? vf::handle_enqueue_chunk(h, kChunk) : vf::handle_enqueue_steps(h, w.enqueued, n);
+  h->af.share = 0;
+  if (rc) return rc;
   w.enqueued += n;
   const int slot = (w.head + w.inflight) % kInFlight;
   cudaError_t e = cudaMemcpyAsync(slot_rec(b->slots[w.member], slot), h->rec, sizeof(vf::StepRecord),

@@ -40,6 +40,7 @@ struct vf_handle {
   int chunk_k = 0;                        // its step count; 0: recapture
   int plain_chunks = 0;                   // chunks run without a graph so far
   void* chunk_u0 = nullptr;               // U[0] when captured (the buffers swap between calls)
+  int chunk_share = 0;                    // StepArgs::share it was captured with
 };
 
 namespace vf {

@@ -27,11 +27,6 @@ template <typename T> struct MarchSeg {
   static constexpr int flux = 40;
   static constexpr int stage = 24;
 };
-// Warps per SM below which a launch is bound by the latency of one warp's rows
-// (1.2 us a row in the flux pass, 2 us in the stage pass) and not by
-// instruction issue.
-constexpr int kMarchWarpsPerSM = 16;
-
 template <typename T>
 cudaError_t configure_impl() {
   cudaError_t e = cudaSuccess;
@@ -105,16 +100,26 @@ cudaError_t ensemble_max_clusters_impl(int csize, int variant, int* out) {
   return cudaOccupancyMaxActiveClusters(out, k_ensemble<T, 1>, &cfg);
 }
 
-// Segment length of one launch: the shortest that leaves kMarchWarpsPerSM warps
-// on each of the 152 SMs, and at most `longest`. With 40 and 24 rows at every
-// size, a 200x120 grid had 24 and 40 warps on the whole GPU: 51 and 57 us a
-// pass, 5.6 ms for a request of 40 steps instead of 1.7; 1021x511 cells 52 and
-// 62 us a pass, 3.0 ms per 24 steps instead of 1.35 (8 / 16 / 24 / 32 warps:
-// 1.87 / 1.35 / 1.36 / 1.32). From about 2400^2 cells on nothing changes.
+// Segment length of one launch: the shortest whose blocks are resident all at
+// once, blocks_per_sm on each of the 152 SMs, and at most `longest`. A launch of
+// fewer warps is bound by the latency of one warp's rows (1.2 us a row in the flux
+// pass, 2 us in the stage pass), one of a second wave by that wave. With 40 and 24
+// rows at every size, a 200x120 grid had 24 and 40 warps on the whole GPU: 51 and
+// 57 us a pass, 5.6 ms for a request of 40 steps instead of 1.7. us per step with
+// segments for 8 / 16 / 28 / 40 warps per SM, the lean form (28 to 32 are resident):
+// 997x753 77 / 53 / 49 / 51, 1021x511 - / 48 / 43 / 45, 1500x1100 107 / 91 / 81 / 83,
+// 2048^2 193 / 195 / 184 / 186; the general form at 8 / 16 / 24 / 40 (24 are
+// resident): 997x753 82 / 58 / 54 / 55, 1500x1100 120 / 105 / 95 / 92. From about
+// 2400^2 cells on nothing changes. Launches of `share` simulations at once fill the
+// GPU together: each takes its part of the wave, in longer segments that recompute
+// fewer halo rows.
 template <typename T>
-int march_seg(const Geom<T>& g, int longest) {
-  const long long nstrips = (g.nx + MOUT - 1) / MOUT, warps = 152LL * kMarchWarpsPerSM;
-  const long long rows = (nstrips * g.ny + warps - 1) / warps;
+int march_seg(const StepArgs<T>& a, int longest, int blocks_per_sm) {
+  const Geom<T>& g = a.g;
+  const long long nstrips = (g.nx + MOUT - 1) / MOUT;
+  const long long units = 152LL * MWPB * blocks_per_sm / (a.share > 1 ? a.share : 1);
+  long long rows = (nstrips * g.ny + units - 1) / units;
+  while (rows < longest && nstrips * ((g.ny + rows - 1) / rows) > units) ++rows;
   return (int)(rows < longest ? rows : longest);
 }
 template <typename T>
@@ -184,7 +189,7 @@ void with_march_form(const StepArgs<T>& a, F f) {
 template <typename T>
 cudaError_t launch_flux_impl(const StepArgs<T>& a, const T* Uin, int parity, cudaStream_t st) {
   if (a.variant == 0) {
-    const int seg = march_seg(a.g, MarchSeg<T>::flux);
+    const int seg = march_seg(a, MarchSeg<T>::flux, MarchFluxBlocks<T>::resident);
     with_march_form(a, [&](auto o, auto gen, auto cb) {
       k_flux_march<T, decltype(o), decltype(gen)::value, decltype(cb)::value>
           <<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, a.rec, parity, seg);
@@ -213,7 +218,8 @@ cudaError_t launch_stage_impl(const StepArgs<T>& a, const T* Uin, T* Uout, int p
     return cudaGetLastError();
   }
   if (a.variant == 0) {
-    const int seg = march_seg(a.g, MarchSeg<T>::stage);
+    const int seg = march_seg(a, MarchSeg<T>::stage,
+                              a.general ? MarchStageBlocks<T>::resident_general : MarchStageBlocks<T>::resident);
     with_march_form(a, [&](auto o, auto gen, auto cb) {
       k_stage_march<T, decltype(o), decltype(gen)::value, decltype(cb)::value>
           <<<march_blocks(a.g, seg), MW * MWPB, 0, st>>>(a.g, a.p, Uin, a.B, a.L, a.S, Uout, a.rec, parity, seg);
