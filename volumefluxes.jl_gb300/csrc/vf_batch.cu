@@ -532,11 +532,17 @@ int pack_pump(vf_batch* b, Pack& k, bool late) {
   return VF_OK;
 }
 
+bool fed(const vf_batch* b) {  // nothing left to enqueue
+  return b->pack.live == 0 && std::all_of(b->wide.begin(), b->wide.end(), [](const Wide& w) { return w.done; });
+}
+
 // Retire finished chunks of the pack and of every wide member, keep kInFlight queued.
 int pump(vf_batch* b) {
   if (b->wide.empty() && b->pack.members.empty()) return VF_OK;
   std::lock_guard<std::mutex> lk(b->mu);
   if (b->feed_rc) return bfail(b, b->feed_rc, b->feed_err);
+  if (fed(b)) return VF_OK;
+  if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, VF_ECUDA, "cudaSetDevice failed");
   const double elapsed =
       std::chrono::duration<double>(std::chrono::steady_clock::now() - b->start).count();
   const bool late = elapsed > b->time_limit_s;
@@ -578,10 +584,6 @@ int pump(vf_batch* b) {
       if (int rc = wide_enqueue(b, w)) return bfail(b, rc, "wide member launch: " + b->hs[w.member]->err);
   }
   return VF_OK;
-}
-
-bool fed(const vf_batch* b) {  // nothing left to enqueue
-  return b->pack.live == 0 && std::all_of(b->wide.begin(), b->wide.end(), [](const Wide& w) { return w.done; });
 }
 
 // Feeds the batch while the caller is elsewhere. With the default threshold members

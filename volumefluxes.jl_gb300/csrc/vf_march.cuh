@@ -338,11 +338,11 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
 template <typename T> struct MarchStageBlocks {
   static constexpr int value = sizeof(T) == 4 ? VF_MARCH_STAGE_BLOCKS_F32 : 1;
   static constexpr int general = sizeof(T) == 4 ? 6 : 1;
-  static constexpr int resident = sizeof(T) == 4 ? value : 2, resident_general = sizeof(T) == 4 ? general : 2;
+  static constexpr int resident = sizeof(T) == 4 ? value : 4, resident_general = sizeof(T) == 4 ? general : 4;
 };
 template <typename T> struct MarchFluxBlocks {
   static constexpr int value = sizeof(T) == 4 ? VF_MARCH_FLUX_BLOCKS_F32 : 1;
-  static constexpr int resident = sizeof(T) == 4 ? value : 2;
+  static constexpr int resident = sizeof(T) == 4 ? value : 4;
 };
 
 // GEN: NoReconstruction and time- or cell-dependent sources as well (the ghost
