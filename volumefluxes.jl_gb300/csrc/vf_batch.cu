@@ -388,7 +388,7 @@ int wide_enqueue(vf_batch* b, Wide& w) {
 constexpr int kPackChunk = 8;  // steps per chunk of a pack
 
 // The block map of the pack's live members, uploaded in stream order.
-int pack_map(vf_batch* b, Pack& k) {
+int pack_map(vf_batch* b, Pack& k) try {
   std::vector<vf::PackBlock> map;
   for (size_t i = 0; i < k.members.size(); ++i) {
     if (k.done[i]) continue;
@@ -409,6 +409,8 @@ int pack_map(vf_batch* b, Pack& k) {
   k.live_at_map = k.live;
   k.remap = false;
   return e == cudaSuccess ? VF_OK : VF_ECUDA;
+} catch (const std::bad_alloc&) {
+  return VF_ENOMEM;
 }
 
 int pack_enqueue(vf_batch* b, Pack& k) {
@@ -432,7 +434,7 @@ int pack_enqueue(vf_batch* b, Pack& k) {
   return VF_OK;
 }
 
-int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts) {
+int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts) try {
   const size_t n = k.members.size();
   cudaMemPool_t pool = vf::device_pool(b->device);
   bool ok = pool && cudaStreamCreateWithFlags(&k.stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -482,6 +484,8 @@ int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts)
   for (int c = 0; c < kInFlight && k.enqueued < b->max_steps; ++c)
     if (int rc = pack_enqueue(b, k)) return rc;
   return VF_OK;
+} catch (const std::bad_alloc&) {
+  return VF_ENOMEM;
 }
 
 void pack_finish(vf_batch* b, Pack& k, size_t j, const vf::StepRecord& r, long long end, int status) {
@@ -595,7 +599,11 @@ void feed(vf_batch* b) {
   g_feeding = true;
   if (cudaSetDevice(b->device) != cudaSuccess) return;
   while (!b->stop) {
-    const int rc = pump(b);
+    int rc = VF_ENOMEM;
+    try {
+      rc = pump(b);
+    } catch (...) {  // no memory for an error's text
+    }
     {
       std::lock_guard<std::mutex> lk(b->mu);
       b->feed_rc = rc;
