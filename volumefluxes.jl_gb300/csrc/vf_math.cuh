@@ -463,7 +463,7 @@ __device__ __forceinline__ void side_flux(const Phys<T>& p, T h, T hu, T hv, T& 
 }
 
 // One side of a Float32 face without branches: a dry side takes depth and
-// reciprocal depth zero, so its flux and eigenvalues come out as zeros. wet: the
+// velocities zero, so its flux and eigenvalues come out as zeros. wet: the
 // side's depth exceeds the cutoff.
 template <int DIR>
 __device__ __forceinline__ void side_flux_f32(const Phys<float>& p, bool wet, float h, float u, float v,
@@ -497,8 +497,9 @@ __device__ __forceinline__ void cu_face_f32(const Phys<float>& p, float mh, floa
   // h* = max(h, min(h^2 / (2 kappa) + kappa/2, kappa)) for h > 0 (src/equations/equation.jl:40-62)
   const float hm = fmaxf(mh, fminf(mh * mh * p.half_over_kappa + p.kappa * 0.5f, p.kappa));
   const float hp = fmaxf(ph, fminf(ph * ph * p.half_over_kappa + p.kappa * 0.5f, p.kappa));
-  const float rm = wm ? A::rcp(hm) : 0.f, rp = wp ? A::rcp(hp) : 0.f;
-  float mu = mhu * rm, mv = mhv * rm, pu = phu * rp, pv = phv * rp;
+  const float rm = A::rcp(hm), rp = A::rcp(hp);
+  // selects, not products with zero: a dry side's momentum may be infinite or NaN
+  float mu = wm ? mhu * rm : 0.f, mv = wm ? mhv * rm : 0.f, pu = wp ? phu * rp : 0.f, pv = wp ? phv * rp : 0.f;
   const bool nm = wm && mh < p.near_dry, np = wp && ph < p.near_dry;
   if (nm || np) {  // thin films take the Float64 quotient's bits
     if (nm) {
@@ -517,12 +518,24 @@ __device__ __forceinline__ void cu_face_f32(const Phys<float>& p, float mh, floa
   const float aminus = fminf(fminf(ep2, em2), 0.f);
   const float d = aplus - aminus;
   const bool waves = !(d < p.kappa);
-  const float R = waves ? A::rcp(d) : 0.f;
+  const float R = waves || !SPEED ? A::rcp(d) : 0.f;
   const float q = (aplus * aminus) * R;
-  F0 = (aplus * fm0 - aminus * fp0) * R + q * (ph - mh);
-  F1 = (aplus * fm1 - aminus * fp1) * R + q * (phu - mhu);
-  F2 = (aplus * fm2 - aminus * fp2) * R + q * (phv - mhv);
-  if (SPEED) speed = waves && !(mh < p.cutoff && ph < p.cutoff) ? fmaxf(aplus, -aminus) : 0.f;
+  const float g0 = (aplus * fm0 - aminus * fp0) * R + q * (ph - mh);
+  const float g1 = (aplus * fm1 - aminus * fp1) * R + q * (phu - mhu);
+  const float g2 = (aplus * fm2 - aminus * fp2) * R + q * (phv - mhv);
+  // No waves, no flux, whatever the values are: zero times a difference that is
+  // infinite or NaN would not be zero. The two forms are the faster one of either
+  // pass (us per 4096^2 wet/dry launch, flux and stage: assignment 253 and 385,
+  // selects 262 and 373; selects around the whole expressions 280 and 389).
+  if constexpr (SPEED) {
+    F0 = g0, F1 = g1, F2 = g2;
+    if (!waves) F0 = F1 = F2 = 0.f;
+    speed = waves ? fmaxf(aplus, -aminus) : 0.f;  // waves: one side at least is wet
+  } else {
+    F0 = waves ? g0 : 0.f;
+    F1 = waves ? g1 : 0.f;
+    F2 = waves ? g2 : 0.f;
+  }
 }
 
 // Central-upwind flux across one face, src/numericalflux/swe/centralupwind.jl:48-77.
