@@ -304,6 +304,11 @@ void destroy_batch(vf_batch* b) {
   if (!b) return;
   b->stop = true;
   if (b->feeder.joinable()) b->feeder.join();
+  // After an error clusters and chunks may still run: they read the descriptors and
+  // write states, result slots and record copies, all handed on below.
+  for (cudaStream_t s : b->streams) cudaStreamSynchronize(s);
+  for (const Wide& w : b->wide)
+    if (!w.done) cudaStreamSynchronize(b->hs[w.member]->stream);  // the handle of one that is done may be gone
   if (b->setup) {
     cudaFreeAsync(b->items_d[0], b->setup);
     cudaFreeAsync(b->items_d[1], b->setup);
@@ -722,7 +727,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     for (int k = 0; rc == VF_OK && k < kInFlight && w.enqueued < w.max_steps; ++k) rc = wide_enqueue(b, w);
     if (rc) {
       cudaGetLastError();
-      for (Wide& x : b->wide) cudaStreamSynchronize(hs[x.member]->stream);
       const std::string msg = std::string("wide member start: ") + h->err;
       destroy_batch(b);
       return bfail(nullptr, rc ? rc : VF_ECUDA, msg);
@@ -738,7 +742,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     cudaStream_t s = nullptr;
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
       cudaGetLastError();
-      for (Wide& x : b->wide) cudaStreamSynchronize(hs[x.member]->stream);
       destroy_batch(b);
       return bfail(nullptr, VF_ECUDA, "stream creation failed");
     }
@@ -752,7 +755,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
   if (e == cudaSuccess) e = cudaMemsetAsync(b->epoch_d, 0, sizeof(unsigned long long), b->setup);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    for (Wide& x : b->wide) cudaStreamSynchronize(hs[x.member]->stream);
     destroy_batch(b);
     return bfail(nullptr, VF_ENOMEM, "batch scratch allocation failed");
   }
@@ -798,7 +800,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
   if (e == cudaSuccess) e = cudaStreamSynchronize(b->setup);
   if (e != cudaSuccess) {
     cudaGetLastError();
-    for (Wide& x : b->wide) cudaStreamSynchronize(hs[x.member]->stream);
     destroy_batch(b);
     return bfail(nullptr, VF_ECUDA, std::string("batch descriptors: ") + cudaGetErrorString(e));
   }
@@ -813,9 +814,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
                                            gr.variant, limit_ns, b->streams[g]);
     if (e != cudaSuccess) {
       cudaGetLastError();
-      // Launches already issued run to completion before anything is freed.
-      for (size_t k = 0; k < g; ++k) cudaStreamSynchronize(b->streams[k]);
-      for (Wide& x : b->wide) cudaStreamSynchronize(hs[x.member]->stream);
       destroy_batch(b);
       return bfail(nullptr, VF_ECUDA, std::string("ensemble launch: ") + cudaGetErrorString(e));
     }
