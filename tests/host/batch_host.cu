@@ -170,9 +170,31 @@ static void error() {
   }
 }
 
+// A member whose time stands still is stepped on by the chunks in flight: its
+// result is the state and the record after the last of them.
+static void stall() {
+  g_dt = 0;
+  for (long long max_steps : {0LL, 19LL, 16LL, 1LL}) {
+    std::vector<vf_handle*> hs = make(3, 128);
+    std::vector<void*> u0;
+    for (vf_handle* h : hs) u0.push_back(h->U[0]);
+    vf_batch* b = launch(hs, 0, 8, max_steps);
+    CHECK(vf_batch_wait(b) == VF_OK);
+    for (int i = 0; i < 3; ++i) {
+      int64_t steps = 0;
+      double t = 1, dt = 1;
+      CHECK(vf_batch_collect(b, i, &t, &steps, &dt, nullptr) == VF_OK);
+      CHECK(steps == hs[i]->rec->n_done && t == 0 && dt == 0);
+      CHECK(hs[i]->U[steps & 1] == u0[i]);
+    }
+    CHECK(vf_batch_free(b) == VF_OK);
+  }
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "error") error();
+  else if (what == "stall") stall();
   else return 2;
   return 0;
 }

@@ -575,7 +575,10 @@ int pump(vf_batch* b) {
         break;
       }
       if (r.t[k & 1] == w.last_t && k > 0) {  // a whole chunk without progress
-        wide_finish(b, w, r, k, vf::kEnsStalled);
+        // Later chunks still step it: its result is the last one's.
+        if (cudaStreamSynchronize(b->hs[w.member]->stream) != cudaSuccess) return bfail(b, VF_ECUDA, "wide member");
+        const int last = w.inflight > 0 ? (w.head + w.inflight - 1) % kInFlight : slot;
+        wide_finish(b, w, *slot_rec(b->slots[w.member], last), w.chunk_end[last], vf::kEnsStalled);
         break;
       }
       w.last_t = r.t[k & 1];
