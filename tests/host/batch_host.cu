@@ -191,10 +191,29 @@ static void stall() {
   }
 }
 
+// Batches of thousands of members are launched while the feeder of another one
+// reads its members' records (run under the thread sanitizer).
+static void slots() {
+  vf_batch* first = launch({make(128)}, 0, 1e9);
+  std::vector<vf_batch*> more;
+  for (int k = 0; k < 5; ++k) {
+    more.push_back(launch(make(3000, 8), 0, 1));
+    std::this_thread::sleep_for(std::chrono::milliseconds(5));
+  }
+  for (vf_batch* b : more) CHECK(vf_batch_free(b) == VF_OK);
+  {
+    LOCK;
+    g_dt = 1e9;
+  }
+  CHECK(left_alone(first, 1));
+  CHECK(vf_batch_free(first) == VF_OK);
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "error") error();
   else if (what == "stall") stall();
+  else if (what == "slots") slots();
   else return 2;
   return 0;
 }

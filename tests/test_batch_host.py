@@ -35,3 +35,11 @@ def driver(tmp_path_factory):
 def test_batch_host(driver, scenario):
     r = subprocess.run([str(driver), scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+def test_feeder_and_launches_share_no_table(tmp_path):
+    driver = compile_driver(tmp_path, "-fsanitize=thread")
+    r = subprocess.run([str(driver), "slots"], capture_output=True, text=True, timeout=300)
+    if "unexpected memory mapping" in r.stderr:
+        pytest.skip("the thread sanitizer does not start under this kernel's address layout")
+    assert r.returncode == 0 and "data race" not in r.stderr, r.stdout + r.stderr[-6000:]

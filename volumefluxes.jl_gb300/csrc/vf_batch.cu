@@ -76,6 +76,17 @@ struct Pack {
   long long chunk_end[3] = {0, 0, 0};
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
 };
+// A slot holds the result a cluster writes (res) and, for wide and packed members,
+// the step-record copies of the chunks in flight. A batch keeps its slots' addresses:
+// its feeder reads them while other batches take slots from the table.
+struct Slot {
+  vf::EnsResult res;
+  vf::StepRecord rec[3];
+};
+struct SlotRef {
+  Slot* host;
+  Slot* dev;  // the same memory's device address
+};
 }  // namespace
 
 struct vf_batch {
@@ -89,7 +100,7 @@ struct vf_batch {
   double time_limit_s = 0;
   std::vector<vf_handle*> hs;
   std::vector<cudaStream_t> streams;
-  std::vector<int> slots;          // result slot of simulation i
+  std::vector<SlotRef> slots;      // result slot of simulation i
   std::vector<char> collected;
   void* items_d[2] = {nullptr, nullptr};  // EnsItem<double>[], EnsItem<float>[]
   int* order_d = nullptr;
@@ -116,22 +127,15 @@ int bfail(vf_batch* b, int code, const std::string& msg) {
 }
 
 // ---- result slots: pinned, device-mapped, never freed ---------------------
-// A slot holds the result a cluster writes (res) and, for wide and packed members,
-// the step-record copies of the chunks in flight.
-struct Slot {
-  vf::EnsResult res;
-  vf::StepRecord rec[3];
-};
-
 constexpr int kSlab = 4096;
 std::mutex g_slot_mu;
-std::vector<Slot*> g_slabs;  // host pointers
-std::vector<Slot*> g_slabs_d;
-std::vector<int> g_free_slots;
+size_t g_slots = 0;                // in all slabs
+std::vector<SlotRef> g_free_slots;  // room for every slot is reserved
 
-int acquire_slots(int n, std::vector<int>& out, std::string& err) {
+int acquire_slots(int n, std::vector<SlotRef>& out, std::string& err) try {
   std::lock_guard<std::mutex> lk(g_slot_mu);
   while ((int)g_free_slots.size() < n) {
+    g_free_slots.reserve(g_slots + kSlab);
     void* p = nullptr;
     if (cudaHostAlloc(&p, sizeof(Slot) * kSlab, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
       cudaGetLastError();
@@ -144,30 +148,29 @@ int acquire_slots(int n, std::vector<int>& out, std::string& err) {
       err = "mapped result slab has no device address";
       return VF_ECUDA;
     }
-    const int base = (int)g_slabs.size() * kSlab;
-    g_slabs.push_back(static_cast<Slot*>(p));
-    g_slabs_d.push_back(static_cast<Slot*>(d));
-    for (int i = kSlab - 1; i >= 0; --i) g_free_slots.push_back(base + i);
+    g_slots += kSlab;
+    for (int i = kSlab - 1; i >= 0; --i)
+      g_free_slots.push_back(SlotRef{static_cast<Slot*>(p) + i, static_cast<Slot*>(d) + i});
   }
-  out.resize(n);
-  for (int i = 0; i < n; ++i) {
-    out[i] = g_free_slots.back();
-    g_free_slots.pop_back();
-  }
+  out.assign(g_free_slots.end() - n, g_free_slots.end());
+  g_free_slots.resize(g_free_slots.size() - n);
   return VF_OK;
+} catch (const std::bad_alloc&) {
+  err = "no host memory";  // short enough to need none
+  return VF_ENOMEM;
 }
 
-void release_slots(const std::vector<int>& s) {
+void release_slots(const std::vector<SlotRef>& s) {
   std::lock_guard<std::mutex> lk(g_slot_mu);
-  for (int v : s) g_free_slots.push_back(v);
+  for (const SlotRef& v : s) g_free_slots.push_back(v);
 }
 
-vf::EnsResult* slot_host(int s) { return &(g_slabs[s / kSlab] + s % kSlab)->res; }
-vf::EnsResult* slot_dev(int s) { return &(g_slabs_d[s / kSlab] + s % kSlab)->res; }
-vf::StepRecord* slot_rec_dev(int s, int k) { return &(g_slabs_d[s / kSlab] + s % kSlab)->rec[k]; }
-vf::StepRecord* slot_rec(int s, int k) { return &(g_slabs[s / kSlab] + s % kSlab)->rec[k]; }
+vf::EnsResult* slot_host(const SlotRef& s) { return &s.host->res; }
+vf::EnsResult* slot_dev(const SlotRef& s) { return &s.dev->res; }
+vf::StepRecord* slot_rec(const SlotRef& s, int k) { return &s.host->rec[k]; }
+vf::StepRecord* slot_rec_dev(const SlotRef& s, int k) { return &s.dev->rec[k]; }
 
-int slot_done(int s) { return __atomic_load_n(&slot_host(s)->done, __ATOMIC_ACQUIRE); }
+int slot_done(const SlotRef& s) { return __atomic_load_n(&slot_host(s)->done, __ATOMIC_ACQUIRE); }
 
 // ---- cluster sizing ---------------------------------------------------------
 struct Opts {
