@@ -209,11 +209,34 @@ static void slots() {
   CHECK(vf_batch_free(first) == VF_OK);
 }
 
+// A batch left alone gets on while a thread of the caller captures in the global
+// mode, and its calls do not end that capture.
+static void capture() {
+  fake::device_runs = false;
+  std::vector<vf_handle*> hs = make(9, 70);  // a pack
+  hs.push_back(make(300));                   // launches of their own
+  hs.push_back(make(8));                     // a cluster
+  vf_batch* b = launch(hs, 0, 40);
+  {
+    LOCK;
+    fake::capturing = fake::device_runs = true;
+  }
+  int32_t done = 0;
+  CHECK(vf_batch_poll(b, &done) == VF_OK);
+  CHECK(left_alone(b, 10));
+  CHECK(vf_batch_poll(b, &done) == VF_OK);
+  CHECK(vf_batch_wait(b) == VF_OK);
+  CHECK(fake::refused == 0);
+  fake::capturing = false;
+  CHECK(vf_batch_free(b) == VF_OK);
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   if (what == "error") error();
   else if (what == "stall") stall();
   else if (what == "slots") slots();
+  else if (what == "capture") capture();
   else return 2;
   return 0;
 }

@@ -31,7 +31,7 @@ def driver(tmp_path_factory):
     return compile_driver(tmp_path_factory.mktemp("batch"))
 
 
-@pytest.mark.parametrize("scenario", ["error", "stall"])
+@pytest.mark.parametrize("scenario", ["error", "stall", "capture"])
 def test_batch_host(driver, scenario):
     r = subprocess.run([str(driver), scenario], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr

@@ -303,8 +303,19 @@ vf::EnsItem<T> make_item(vf_handle* h, const vf::StepArgs<T>& a, double t0, doub
   return it;
 }
 
+// While any thread captures a graph in the global mode, event queries, waits and
+// pool allocations of the other threads are refused and end that capture. The calls
+// that feed a batch touch its own streams alone, so they opt out for their duration:
+// the feeder runs beside whatever its caller does.
+struct BesideCaptures {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 void destroy_batch(vf_batch* b) {
   if (!b) return;
+  const BesideCaptures beside;
   b->stop = true;
   if (b->feeder.joinable()) b->feeder.join();
   // After an error clusters and chunks may still run: they read the descriptors and
@@ -551,6 +562,7 @@ bool fed(const vf_batch* b) {  // nothing left to enqueue
 // Retire finished chunks of the pack and of every wide member, keep kInFlight queued.
 int pump(vf_batch* b) {
   if (b->wide.empty() && b->pack.members.empty()) return VF_OK;
+  const BesideCaptures beside;
   std::lock_guard<std::mutex> lk(b->mu);
   if (b->feed_rc) return bfail(b, b->feed_rc, b->feed_err);
   if (fed(b)) return VF_OK;
@@ -863,6 +875,7 @@ int vf_batch_collect(vf_batch* b, int32_t i, double* t_out, int64_t* steps_out, 
 
 int vf_batch_wait(vf_batch* b) {
   if (!b) return bfail(b, VF_EINVAL, "NULL batch");
+  const BesideCaptures beside;
   if (cudaSetDevice(b->device) != cudaSuccess) return bfail(b, VF_ECUDA, "cudaSetDevice failed");
   for (;;) {  // wide members and packs need the host to feed them
     if (int rc = pump(b)) return rc;
