@@ -209,6 +209,10 @@ bool busy(const vf_server* s) {
 // The engine thread: complete, admit, launch, feed wide members; about every
 // 100 us while anything runs, asleep otherwise.
 void engine_loop(vf_server* s) {
+  // A graph that some thread of the caller captures in the global mode (torch's
+  // default) would refuse this thread's waits and copies, and be ended by them.
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
   cudaSetDevice(s->device);
   std::unique_lock<std::mutex> lk(s->mu);
   while (!s->stop) {
