@@ -296,14 +296,17 @@ void make_tma_maps(vf_handle* h) {
 // for their ghost, source and reconstruction branches) for everything else;
 // with tiles a 997x753 periodic grid with time-dependent sources took 37 + 62 us
 // a step. Float64 runs tiles; VF_KERNELS=march gives it the marching kernels.
+// VF_KERNELS=march64: Float32 with the 64-bit offsets of planes of 4 GB and more.
 void select_variants(vf_handle* h) {
   const bool lean = h->cfg.bc == VF_BC_WALL && h->ad.p.rec_none == 0 && h->ad.p.any_dynamic == 0;
   h->ad.variant = 1;
   h->af.variant = 0;
   h->ad.general = h->af.general = lean ? 0 : 1;
+  h->ad.far = h->af.far = 0;
   if (const char* kv = std::getenv("VF_KERNELS")) {
     if (std::strcmp(kv, "tile") == 0) h->ad.variant = h->af.variant = 1;
     if (std::strcmp(kv, "march") == 0) h->ad.variant = 0;
+    if (std::strcmp(kv, "march64") == 0) h->af.far = 1;
   }
 }
 

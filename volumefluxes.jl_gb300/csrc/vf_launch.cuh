@@ -24,6 +24,7 @@ struct StepArgs {
   int rk2;
   int variant;  // 0: column-marching kernels, 1: shared-memory tile kernels
   int general;  // marching: the kernels for every boundary kind, reconstruction and source (Float32)
+  int far;      // marching: 64-bit offsets where 32-bit ones would do
   int share;    // marching: simulations that share the GPU with this launch, 0 or 1: none (march_seg)
   const T* B;
   T* L;

@@ -174,7 +174,7 @@ template <typename T, typename F>
 void with_march_form(const StepArgs<T>& a, F f) {
   using u32 = unsigned;
   using u64 = unsigned long long;
-  const bool small = plane_fits_u32<T>(a.g);
+  const bool small = plane_fits_u32<T>(a.g) && !a.far;
   if constexpr (sizeof(T) == 8) {
     if (a.general) f(u64{}, std::true_type{}, std::integral_constant<int, 2>{});
     else f(u64{}, std::false_type{}, std::integral_constant<int, 2>{});
