@@ -53,7 +53,7 @@ def nvcc() -> str:
 
 
 def sources() -> list[Path]:
-    return sorted(list(CSRC.glob("*.cu")) + list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h")))
+    return sorted(f for pattern in ("*.cu", "*.cuh", "*.h") for f in (*CSRC.glob(pattern), *INCLUDE.glob(pattern)))
 
 
 def up_to_date() -> bool:
