@@ -19,7 +19,7 @@
 //                     rounded reciprocal and Markstein's residual took 3 of
 //                     them per quotient and 5 per divisor;
 //  square_root        RN(sqrt(x)) the same way from a Float32 reciprocal root;
-//  cube_root_seed     cbrt within an ulp or two from a Float32 seed and one
+//  cube_root_seed     cbrt within a few ulps from a Float32 seed and one
 //                     Taylor step in 7 Float64 operations.
 //
 // All of them return the IEEE result for every operand: operands outside the
@@ -84,7 +84,12 @@ VF_XFN float ffma(float a, float b, float c) { return std::fma(a, b, c); }
 VF_XFN float fmulr(float a, float b) { return a * b; }
 VF_XFN float frcp(float x) { return ffrom(fbits(1.0f / x) + (u32)(VF_SEED_ULPS)); }
 VF_XFN float frsqrt(float x) { return ffrom(fbits((float)(1.0 / std::sqrt((double)x))) + (u32)(VF_SEED_ULPS)); }
-VF_XFN float fmcbrt(float x) { return ffrom(fbits((float)(1.0 / std::cbrt((double)x))) + (u32)(8 * VF_SEED_ULPS)); }
+#ifndef VF_CBRT_SEED_ERROR  // relative
+#define VF_CBRT_SEED_ERROR 0
+#endif
+VF_XFN float fmcbrt(float x) {
+  return ffrom(fbits((float)((1.0 + VF_CBRT_SEED_ERROR) / std::cbrt((double)x))) + (u32)(8 * VF_SEED_ULPS));
+}
 VF_XFN double dfma(double a, double b, double c) { return std::fma(a, b, c); }
 VF_XFN double dmul(double a, double b) { return a * b; }
 VF_XFN double ddiv(double a, double b) { return a / b; }
@@ -232,9 +237,11 @@ VF_XFN double square_root(double x) {
   return from_bits((u64)s - (1ull << 52) + ((u64)(e << 20) << 32));
 }
 
-// cbrt(t) for t in [1, 8), within about an ulp: with w ~ t^(-1/3) and
-// e = 1 - t w^3, cbrt(t) = t w^2 (1 - e)^(-2/3), whose Taylor series after
-// e^2 leaves 40/81 e^3 < 2^-56.
+// cbrt(t) for t in [1, 8), within 5.3 units of 2^-53 relative: with w ~ t^(-1/3)
+// and e = 1 - t w^3, cbrt(t) = t w^2 (1 - e)^(-2/3). A w off by 2^-19 gives
+// |e| < 3.01 2^-19, and the Taylor series after e^2 leaves 40/81 e^3 < 0.85 2^-53;
+// the roundings of t w, w^2 and c add 2 units through c and 4/3 through e, the
+// last sum another. cr_cbrt finds the nearest double by exact comparisons.
 VF_XFN double cube_root_seed(double t) {
   const u64 v = bits(t);
   // Float32 value of t by its bits (a conversion instruction runs on the FP64 pipe)

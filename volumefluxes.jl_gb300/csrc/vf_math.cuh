@@ -105,8 +105,8 @@ struct Arith<float> {
 };
 
 // ---------------------------------------------------------------------------
-// Correctly rounded cube root (Float64). A seed within an ulp or two is
-// corrected with an exact integer comparison against the rounding midpoints, so
+// Correctly rounded cube root (Float64). A seed within a few ulps (eight at most)
+// is corrected with an exact integer comparison against the rounding midpoints, so
 // the result is the nearest double regardless of the seed's last-bit error; the
 // CPU oracle computes the same unique value.
 __device__ __forceinline__ void cube_u55(uint64_t k, uint64_t& w0, uint64_t& w1, uint64_t& w2) {
