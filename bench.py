@@ -107,10 +107,12 @@ def profile_table(tag: str):
 
 def kernel_names(dtype: str) -> dict:
     """Kernels the library runs for this precision (TMA-staged tiles for Float64,
-    marching for Float32; VF_KERNELS and VF_TMA=0 override)."""
+    marching for Float32; VF_KERNELS and VF_TMA=0 override), each as name<type>; a
+    marching kernel's number is its longest segment in rows, which this workload
+    runs at (a launch argument, not a template's)."""
     variant = os.environ.get("VF_KERNELS", "tile" if dtype == "f64" else "march")
     t = "double" if dtype == "f64" else "float"
-    if variant == "march":  # template arguments: rows per segment of each pass
+    if variant == "march":
         return {"flux": f"k_flux_march<{t},40>", "stage": f"k_stage_march<{t},24>"}
     if dtype == "f64" and os.environ.get("VF_TMA", "1") != "0":
         return {"flux": "k_flux_tma<double>", "stage": "k_stage2_tma<double>"}

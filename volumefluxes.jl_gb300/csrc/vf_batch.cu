@@ -215,10 +215,13 @@ long long wide_cells_for(const vf_handle* h, const Opts& o) {
 // Float64 RK2 members of kPackCells interior cells and more are stepped together as
 // a pack (vf_pack.cuh) while they are below kAloneCells, where launches of their
 // own, with TMA staging, are 4% faster (24 members of 200-500^2 cells, 24 steps:
-// 29.6 ms packed up to 512^2, 28.4 ms alone); the smallest are left to clusters. A
-// pack takes about 0.1 ms to set up: below kPackMembers of them each goes alone.
-// All designs give the same Float64 bits, so this may depend on the batch.
-// Makespan in ms, pack / all alone / alone from 8192 cells on, clusters below:
+// 29.6 ms packed up to 512^2, 28.4 ms alone). kPackCells is the smallest size that
+// was measured, 64^2, and a pack still wins there: the size at which clusters take
+// over is not known, it lies below. A pack takes about 0.1 ms to set up: below
+// kPackMembers of them each goes alone. All designs give the same Float64 bits, so
+// this may depend on the batch.
+// Makespan in ms, pack / all alone / alone from 8192 cells on, clusters below (the
+// best of a state's first calls: of the 8 steps the members take four on average):
 //   20 members of 64-224^2, 8 steps: 1.84 / 2.21 / 4.15; 64: 4.97 / 6.27 / 8.14;
 //   8: 1.12 / 1.09 / 2.17; 4: 0.70 / 0.66 / 1.81; 64 of 64-96^2: 2.53 / 3.75 /
 //   3.79; 200 of 64-80^2, 40 steps: 27.8 / 55.7 / 40.6; 4 of those: 2.17 / 1.66 /

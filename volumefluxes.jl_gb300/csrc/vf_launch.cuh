@@ -7,7 +7,7 @@
 #include "vf_march.cuh"
 #include "vf_pack.cuh"
 
-// Float64 step kernels with faithful quotients and multiply-add contraction
+// Float64 step kernels with fused multiply-adds in the face fluxes
 // (vf_f64f.cu, a unit whose kernels live in their own namespace). `args` points
 // to a vf::StepArgs<double>; same contract as vf::launch_step / launch_flux /
 // launch_stage.
@@ -31,7 +31,7 @@ struct StepArgs {
   T* S;
   StepRecord* rec;
   TmaMaps tma;  // Float64 tile kernels: TMA staging when tma.ok and the buffers match
-  int arith;    // Float64 per-step kernels: 0 rounded as the reference, 1 faithful quotients (vf_f64f.cu)
+  int arith;    // Float64 per-step kernels: 0 rounded as the reference, 1 fused multiply-adds (vf_f64f.cu)
 };
 
 // One full step reading Uin, writing Uout; parity selects the record slot.

@@ -325,9 +325,9 @@ __device__ __forceinline__ void flux_march_unit(const Geom<T>& g, const Phys<T>&
 
 // Resident blocks per SM the Float32 kernels are compiled for. The flux pass
 // fits eight (64 registers, no spill); the stage pass runs best at seven (72
-// registers, 92 bytes of spill): 4096^2 wet/dry, four steps, 2.62 ms at 8 / 7
+// registers, 100 bytes of spill): 4096^2 wet/dry, four steps, 2.62 ms at 8 / 7
 // blocks, 2.67 at 8 / 6, 2.71 at 8 / 8 (3.15 before the offsets, the branch-free
-// faces and the shared Float32 dt). Float64 (190 registers) is bound by the FP64
+// faces and the shared Float32 dt; 2.59 at 8 / 7 with the faces' selects). Float64 (190 registers) is bound by the FP64
 // pipe and is left alone.
 #ifndef VF_MARCH_STAGE_BLOCKS_F32
 #define VF_MARCH_STAGE_BLOCKS_F32 7

@@ -7,8 +7,9 @@
 // where launches of their own would pay two launches per member and step, and a
 // cluster leaves a member 16 SMs at most. The tiles are the plain kernels' and
 // give the same bits. Bound by the FP64 pipe where there are enough members, by
-// launches and tails with few: 20 members of 64-224^2 cells, 8 steps, took 4.15 ms
-// as clusters and launches of their own, 1.84 ms packed; 200 of 64-80^2, 40 steps,
+// launches and tails with few: 20 members of 64-224^2 cells, at most 8 steps, took
+// 4.15 ms as clusters and launches of their own, 1.84 ms packed, while they took four
+// steps on average (4.0 ms packed when all take eight); 200 of 64-80^2, 40 steps,
 // 40.6 and 27.8 ms (vf_batch.cu has where the line lies).
 // A member that has ended costs its blocks' empty turns until the host drops it
 // from the map.

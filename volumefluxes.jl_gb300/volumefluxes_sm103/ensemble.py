@@ -2,12 +2,14 @@
 
 The reference advances one Simulator per simulate_to_time call
 (src/simulator.jl:179-212). `simulate_batch` runs that loop for a list of
-simulators at once, each to its own end time with its own CFL dt; on the
-device every simulation is one thread-block cluster that keeps stepping until
-its end time, and the GPU's block scheduler starts the next pending simulation
-whenever a cluster finishes. `BatchRun` is the non-blocking form used by the
-serving loop: launch, poll which simulations have finished, collect them one
-by one while the rest keep running.
+simulators at once, each to its own end time with its own CFL dt. A small
+simulation is one thread-block cluster that keeps stepping until its end time,
+and the GPU's block scheduler starts the next pending one whenever a cluster
+finishes; a large one runs the whole-grid kernels on a stream of its own; eight
+or more mid-size Float64 ones are stepped together by launches that span them
+all. The last two are fed by a host thread of the batch. `BatchRun` is the
+non-blocking form: launch, poll which simulations have finished, collect them
+one by one while the rest keep running.
 """
 from __future__ import annotations
 

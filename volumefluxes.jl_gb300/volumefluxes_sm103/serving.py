@@ -5,7 +5,7 @@ include/volumefluxes_sm103.h). A request carries a scenario (grid, terrain,
 rain, friction), the real type and an end time; the engine admits requests
 oldest-first while their device memory fits the HBM budget, launches each
 poll's admissions as one batch beside the batches still running, and hands the
-final interior state back when the request's cluster finishes. Requests run to
+final interior state back when the request's simulation finishes. Requests run to
 their end time exactly as `simulate_to_time` would run them alone.
 """
 from __future__ import annotations
