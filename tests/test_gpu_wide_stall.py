@@ -1,6 +1,6 @@
 """A batch member whose time stands still (t + dt rounds to t), on launches of its own:
-the result is the state after the steps it reports, also where the last chunk of steps
-is a short one of odd length."""
+it ends with the step that left t unchanged, as a cluster member does, and so does a
+Float32 one whose end time is not a Float32 number."""
 import math
 
 import numpy as np
@@ -25,9 +25,19 @@ def test_a_wide_member_whose_time_stands_still(real, options, max_steps):
     kw = {} if max_steps is None else {"max_steps": max_steps}
     res = E.simulate_batch(sims, [2.0 ** 70, 0.1, 0.1], options=options, **kw)
     assert res[0].status == N.VF_BATCH_STALLED and res[0].t == 2.0 ** 66
-    assert max_steps is None or res[0].steps <= max_steps
-    for _ in range(res[0].steps):
-        vf.perform_step(ref, math.inf)
+    assert res[0].steps == 1
+    vf.perform_step(ref, math.inf)
     assert res[0].last_dt == vf.current_timestep(ref)
     for a, b in zip(interior(sims[0]), interior(ref)):
         assert np.array_equal(a, b)
+
+
+def test_an_end_time_between_two_float32_numbers():
+    """The same steps, t and status on launches of its own as in a cluster."""
+    got = []
+    for options in (E.BatchOptions(wide_cells=1), E.BatchOptions(wide_cells=-1)):
+        sim = hills_rect(300, 280, B=None, bottom_source=False).build(vf.SM103Backend(np.float32))
+        r, = E.simulate_batch([sim], [0.7], options=options)
+        got.append((r.t, r.steps, r.status))
+    assert got[0] == got[1]
+    assert got[0][2] == N.VF_BATCH_STALLED

@@ -461,7 +461,7 @@ namespace vf {
 int handle_ready(vf_handle* h) { return ensure_ready(h); }
 
 int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep,
-                      long long max_steps) {
+                      long long max_steps, bool stop_stalled) {
   reset_record(h);
   vf::StepRecord* r = h->rec_h;
   r->t[0] = t0;
@@ -471,6 +471,7 @@ int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime
   r->max_ts = maximum_timestep;
   r->endtime = endtime;
   r->max_steps = max_steps > 0 ? max_steps : 0;
+  r->stop_stalled = stop_stalled ? 1 : 0;
   return push_record(h);
 }
 

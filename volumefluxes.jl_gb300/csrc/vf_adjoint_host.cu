@@ -279,7 +279,7 @@ int checkpoint(vf_adjoint* a, int n, const void* U) {
 int forward_cfl(vf_adjoint* a) {
   vf_handle* h = a->h;
   if (int rc = restart(a)) return rc;
-  if (int rc = vf::handle_begin_loop(h, 0.0, INFINITY, 0, -1.0, 0)) return afail(a, rc, "forward step: " + h->err);
+  if (int rc = vf::handle_begin_loop(h, 0.0, INFINITY, 0, -1.0, 0, false)) return afail(a, rc, "forward step: " + h->err);
   for (int n = 0; n < a->n_steps; ++n) {
     if (int rc = checkpoint(a, n, h->U[n & 1])) return rc;
     if (int rc = vf::handle_enqueue_steps(h, n, 1)) return afail(a, rc, "forward step: " + h->err);

@@ -55,14 +55,12 @@ struct Wide {
   int head = 0, inflight = 0;  // chunks head .. head+inflight-1 are in flight; chunk c uses ev/rec slot c % 3
   long long chunk_end[3] = {0, 0, 0};
   cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-  double last_t = 0;
   bool done = false;
 };
 // Members stepped together (vf_pack.cuh).
 struct Pack {
   std::vector<int> members;     // batch indices, in item order
   std::vector<char> done;
-  std::vector<double> last_t;
   int live = 0;
   cudaStream_t stream = nullptr;
   vf::PackItem<double>* items = nullptr;
@@ -70,7 +68,6 @@ struct Pack {
   vf::PackBlock* map = nullptr;
   int n_blocks = 0;
   int live_at_map = 0;          // members the map holds
-  bool remap = false;           // the map holds a member that must not step again
   long long enqueued = 0;
   int head = 0, inflight = 0;   // chunks head .. head+inflight-1; chunk c uses ev/report slot c % 3
   long long chunk_end[3] = {0, 0, 0};
@@ -354,6 +351,12 @@ constexpr int kChunk = 16;    // steps per graph launch of a wide member
 constexpr int kInFlight = 3;  // chunks kept queued per wide member (rides out host stalls)
 constexpr int kPlainChunks = 4;  // chunks a handle runs kernel by kernel before its graph is captured
 
+// How the device loop of a wide or packed member ended, from its record after step k.
+int end_status(const vf::StepRecord& r, long long k, long long max_steps, double endtime) {
+  if (r.stalled) return vf::kEnsStalled;
+  return r.n_done >= max_steps && r.t[k & 1] < endtime ? vf::kEnsMaxSteps : vf::kEnsOk;
+}
+
 // Final result of a wide member from the record copy of its last retired chunk.
 void wide_finish(vf_batch* b, Wide& w, const vf::StepRecord& r, long long k, int status) {
   vf_handle* h = b->hs[w.member];
@@ -429,7 +432,6 @@ int pack_map(vf_batch* b, Pack& k) try {
   // the copy reads a pageable host vector: finish it before the vector goes
   if (e == cudaSuccess) e = cudaStreamSynchronize(k.stream);
   k.live_at_map = k.live;
-  k.remap = false;
   return e == cudaSuccess ? VF_OK : VF_ECUDA;
 } catch (const std::bad_alloc&) {
   return VF_ENOMEM;
@@ -481,6 +483,7 @@ int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts)
     r.endtime = b->endtime[i];
     r.stop_time = std::numeric_limits<double>::infinity();
     r.max_steps = b->max_steps == LLONG_MAX ? 0 : b->max_steps;
+    r.stop_stalled = 1;
     vf::PackItem<double>& it = items[j];
     std::memset(&it, 0, sizeof(it));
     it.g = h->ad.g;
@@ -494,8 +497,6 @@ int pack_start(vf_batch* b, Pack& k, const double* t0, int match, double max_ts)
     for (int c = 0; c < kInFlight; ++c) it.report[c] = slot_rec_dev(b->slots[i], c);
   }
   k.done.assign(n, 0);
-  k.last_t.resize(n);
-  for (size_t j = 0; j < n; ++j) k.last_t[j] = t0[k.members[j]];
   k.live = (int)n;
   ok = cudaMemcpyAsync(k.items, items.data(), sizeof(vf::PackItem<double>) * n, cudaMemcpyHostToDevice, k.stream) ==
        cudaSuccess;
@@ -535,23 +536,14 @@ int pack_pump(vf_batch* b, Pack& k, bool late) {
       if (k.done[j]) continue;
       const int i = k.members[j];
       const vf::StepRecord& r = *slot_rec(b->slots[i], slot);
-      const double t = r.t[end & 1];
       if (!r.active[end & 1])
-        pack_finish(b, k, j, r, end, r.n_done >= b->max_steps && t < b->endtime[i] ? vf::kEnsMaxSteps : vf::kEnsOk);
-      else if (t == k.last_t[j]) {  // a whole chunk without progress
-        // Later chunks still step it: its result is the last one's, and the map
-        // drops it before the next.
-        if (cudaStreamSynchronize(k.stream) != cudaSuccess) return bfail(b, VF_ECUDA, "pack");
-        const int last = k.inflight > 0 ? (k.head + k.inflight - 1) % kInFlight : slot;
-        pack_finish(b, k, j, *slot_rec(b->slots[i], last), k.chunk_end[last], vf::kEnsStalled);
-        k.remap = true;
-      } else if (late && k.inflight == 0)
+        pack_finish(b, k, j, r, end, end_status(r, end, b->max_steps, b->endtime[i]));
+      else if (late && k.inflight == 0)
         pack_finish(b, k, j, r, end, vf::kEnsTimeout);
-      k.last_t[j] = t;
     }
   }
   if (k.live == 0 || late) return VF_OK;
-  if (k.remap || 2 * k.live <= k.live_at_map)  // half of the members have ended: drop their blocks
+  if (2 * k.live <= k.live_at_map)  // half of the members have ended: drop their blocks
     if (int rc = pack_map(b, k)) return bfail(b, rc, "pack map");
   while (k.inflight < kInFlight && k.enqueued < b->max_steps)
     if (int rc = pack_enqueue(b, k)) return bfail(b, rc, "pack launch failed");
@@ -589,17 +581,9 @@ int pump(vf_batch* b) {
       if (r.wait_fault)
         return bfail(b, VF_ECUDA, "wide member: a bounded wait for a TMA tile copy gave up");
       if (!r.active[k & 1]) {
-        wide_finish(b, w, r, k, r.n_done >= w.max_steps && r.t[k & 1] < w.endtime ? vf::kEnsMaxSteps : vf::kEnsOk);
+        wide_finish(b, w, r, k, end_status(r, k, w.max_steps, w.endtime));
         break;
       }
-      if (r.t[k & 1] == w.last_t && k > 0) {  // a whole chunk without progress
-        // Later chunks still step it: its result is the last one's.
-        if (cudaStreamSynchronize(b->hs[w.member]->stream) != cudaSuccess) return bfail(b, VF_ECUDA, "wide member");
-        const int last = w.inflight > 0 ? (w.head + w.inflight - 1) % kInFlight : slot;
-        wide_finish(b, w, *slot_rec(b->slots[w.member], last), w.chunk_end[last], vf::kEnsStalled);
-        break;
-      }
-      w.last_t = r.t[k & 1];
       if (late && w.inflight == 0) {
         wide_finish(b, w, r, k, vf::kEnsTimeout);
         break;
@@ -708,7 +692,6 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
       w.member = i;
       w.max_steps = max_steps > 0 ? max_steps : LLONG_MAX;
       w.endtime = endtime[i];
-      w.last_t = t0[i];
       b->wide.push_back(w);
       continue;
     }
@@ -743,7 +726,7 @@ int vf_batch_launch(vf_handle* const* hs, int32_t n, const double* t0, const dou
     bool ok = true;
     for (cudaEvent_t& e : w.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     int rc = ok ? vf::handle_begin_loop(h, t0[w.member], endtime[w.member], match_endtime, maximum_timestep,
-                                           max_steps)
+                                           max_steps, true)
                 : VF_ECUDA;
     for (int k = 0; rc == VF_OK && k < kInFlight && w.enqueued < w.max_steps; ++k) rc = wide_enqueue(b, w);
     if (rc) {

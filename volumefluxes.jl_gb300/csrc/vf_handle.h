@@ -49,9 +49,10 @@ namespace vf {
 int handle_ready(vf_handle* h);
 // Device-resident time loop of vf_simulate, driven asynchronously: write the
 // loop's record (t0, end time, match_endtime, maximum_timestep < 0: none,
-// max_steps <= 0: none) to the device on the handle's stream.
+// max_steps <= 0: none, stop_stalled: at a step that leaves t unchanged) to the
+// device on the handle's stream.
 int handle_begin_loop(vf_handle* h, double t0, double endtime, int match_endtime, double maximum_timestep,
-                      long long max_steps);
+                      long long max_steps, bool stop_stalled);
 // Copies the step record to the host (h->rec_h) and waits for the stream; an
 // error when a bounded wait of a step gave up.
 int handle_pull_record(vf_handle* h);

@@ -76,6 +76,8 @@ struct StepRecord {
   int explicit_mode;
   int force_dt;        // 1: every step uses forced_dt (a frozen dt sequence)
   int wait_fault;      // set when a bounded wait for a tile copy gave up
+  int stop_stalled;    // device loop: stop after a step that leaves t unchanged (batch members)
+  int stalled;         // set when it did
   double forced_dt;
 };
 
@@ -545,8 +547,10 @@ __device__ __forceinline__ void advance_record(StepRecord* rec, int parity, doub
   rec->t[parity ^ 1] = tn;
   const long long done = rec->n_done + 1;
   rec->n_done = done;
+  const bool still = rec->stop_stalled && tn == rec->t[parity];
+  if (still) rec->stalled = 1;
   const bool more = !rec->explicit_mode && (tn < rec->endtime) && !(tn + dt >= rec->stop_time) &&
-                    !(rec->max_steps > 0 && done >= rec->max_steps);
+                    !(rec->max_steps > 0 && done >= rec->max_steps) && !still;
   rec->active[parity ^ 1] = more ? 1 : 0;
   rec->speed_bits[parity ^ 1][0] = 0ull;
   rec->speed_bits[parity ^ 1][1] = 0ull;
